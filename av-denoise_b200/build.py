@@ -41,8 +41,9 @@ COMMON = [
 # for its reading and fold words, the truemotion stage for its costs and confidences, the exact
 # NLMeans finish for its distances, weights and sums, the colour grain gains for their fit, and the
 # camera model for its fit and composition.
-PER_FILE = {"collab.cu": ["-fmad=false"], "noise_estimate.cu": ["-fmad=false"], "truemotion.cu": ["-fmad=false"],
-            "nlm_exact.cu": ["-fmad=false"], "colour.cu": ["-fmad=false"], "camera.cu": ["-fmad=false"]}
+PER_FILE = {"collab.cu": ["-fmad=false"], "collab_search.cu": ["-fmad=false"], "noise_estimate.cu": ["-fmad=false"],
+            "truemotion.cu": ["-fmad=false"], "nlm_exact.cu": ["-fmad=false"], "colour.cu": ["-fmad=false"],
+            "camera.cu": ["-fmad=false"]}
 
 
 def _sources() -> list[Path]:

@@ -1,11 +1,10 @@
-// NL4D collaborative filter for sm_100a: group search, 2D DCT + Haar hard/pooled threshold,
-// inverse transforms and fixed-point aggregation, one launch per pass.
+// NL4D collaborative filter for sm_100a: 2D DCT + Haar hard/pooled threshold, inverse transforms and
+// fixed-point aggregation, after the group search (collab_search.cu).
 //
 // What it computes (av-denoise-core/src/collab/kernels/fused/mod.rs:170-891): for every reference
-// patch (8x8 on a step-4 grid of the centre frame) the best 8 positions of the centre frame's
-// spatial window (self match pinned first, ties keep the earlier position), optionally grown into
-// volumes along the neighbour frames' motion (fused/trajectory.rs), a 2D DCT per member, a Haar
-// along the stack (or time and volumes), a hard or pooled threshold against lambda x the
+// patch (8x8 on a step-4 grid of the centre frame) the members the search found (the best 8 positions
+// of the centre frame's spatial window, or volumes along the neighbour frames' motion), a 2D DCT per
+// member, a Haar along the stack (or time and volumes), a hard or pooled threshold against lambda x the
 // propagated noise, the inverse transforms, and a Kaiser-tapered fixed-point scatter of every
 // member into its own frame's accumulator region, weighted by 1 / (retained variance).
 //
@@ -24,6 +23,7 @@
 
 #include <cstdint>
 
+#include "collab_group.cuh"
 #include "colour_lookup.cuh"
 #include "kernels.h"
 
@@ -31,59 +31,10 @@ namespace avd {
 
 namespace {
 
-constexpr int P = 8;
-constexpr int STEP = 4;
-constexpr int MAX_K = 8;
-constexpr int kGroups = 16;  // reference patches per CTA
-constexpr int kThreads = kGroups * 8;
-constexpr float kUnfilled = 3.0e38f;
-constexpr float kSelfPin = -1.0e38f;
-constexpr float kReciprocalFloor = 1e-12f;
-constexpr float kAccumClamp = 5.0f;
-constexpr float kWeightGain = 5.0f;
-constexpr float kVarianceFloor = 1.0e-20f;
-constexpr float kFrac1Sqrt2 = 0.70710678118654752440f;
-constexpr int kCurveBins = 16;
+using namespace collab_detail;
 
 // The orthonormal 8-point DCT-II taps, c_row * cos(pi * (2 col + 1) row / 16), in f32.
 __constant__ float c_dct[8][8];
-
-struct GroupCtx {
-    unsigned mask;  // this group's 8 lanes of the warp
-    int sub;        // lane within the group
-};
-
-__device__ __forceinline__ float reduce8(const GroupCtx& g, float v) {
-    v += __shfl_xor_sync(g.mask, v, 1);
-    v += __shfl_xor_sync(g.mask, v, 2);
-    v += __shfl_xor_sync(g.mask, v, 4);
-    return v;
-}
-
-__device__ __forceinline__ uint32_t pack_pos_t(uint32_t x, uint32_t y, uint32_t t) {
-    return (t << 26) | (y << 13) | x;
-}
-
-__device__ __forceinline__ uint32_t clamp_top_left(int v, uint32_t max_pos) {
-    return v < 0 ? 0u : (v > static_cast<int>(max_pos) ? max_pos : static_cast<uint32_t>(v));
-}
-
-// The lane's share of the distance from `ref` (its 8 x C column) to the candidate at (x, y).
-template <int C>
-__device__ __forceinline__ float column_ssd(const float (&ref)[P * C], const float* __restrict__ frame, int width,
-                                            uint32_t x, uint32_t y, int sub) {
-    float s = 0.0f;
-    const float* p = frame + (static_cast<size_t>(y) * width + x + sub) * C;
-#pragma unroll
-    for (int r = 0; r < P; ++r) {
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            float d = ref[r * C + c] - __ldg(p + static_cast<size_t>(r) * width * C + c);
-            s = __fadd_rn(s, __fmul_rn(d, d));
-        }
-    }
-    return s;
-}
 
 __device__ __forceinline__ void dct8_fwd(float (&line)[P]) {
     float s[4], d[4];
@@ -341,316 +292,6 @@ __device__ __forceinline__ int32_t to_fixed(float value, float scale) {
 
 __device__ __forceinline__ int32_t to_fixed_weight(float weight, float scale) {
     return static_cast<int32_t>(roundf(fminf(fmaxf(weight, 0.0f), 1.0f) * scale * kWeightGain));
-}
-
-__device__ __forceinline__ uint32_t covering_lo(uint32_t patch_start, uint32_t blksize, uint32_t step) {
-    const uint32_t overhang = max(patch_start + P, blksize) - blksize;
-    return (overhang + step - 1) / step;
-}
-
-// fused/trajectory.rs (clipped walk): for each neighbour frame the best candidate over one refine
-// rectangle per covering motion block (blocks under c_min skipped, rectangles already searched and
-// positions the group holds skipped), inserted into the volume's sorted tail. COVERS (the covering
-// blocks per axis, ceil(blksize / step)) is a template argument so the rectangles searched so far
-// stay in registers. A skipped candidate can only matter if it would beat the frame's best so far,
-// so the skip test runs for those alone; the winner is the same.
-template <int C, int GF, int FIRST, int COVERS>
-__device__ __forceinline__ void trajectory_search(const GroupCtx& g, const CollabLaunch& a, const float (&anchor)[P * C],
-                                                  uint32_t ax, uint32_t ay, float scale, float (&grid_d)[MAX_K],
-                                                  uint32_t (&grid_pos)[MAX_K]) {
-    constexpr int TAIL = GF - 1;
-    constexpr int RECTS = COVERS * COVERS;
-    const uint32_t max_x = a.width - P, max_y = a.height - P;
-    const uint32_t bx_hi = min(ax / a.blk_step, static_cast<uint32_t>(a.blocks_x - 1));
-    const uint32_t by_hi = min(ay / a.blk_step, static_cast<uint32_t>(a.blocks_y - 1));
-    const uint32_t bx_lo = min(covering_lo(ax, a.blksize, a.blk_step), bx_hi);
-    const uint32_t by_lo = min(covering_lo(ay, a.blksize, a.blk_step), by_hi);
-    for (int t = 0; t < 2 * a.radius; ++t) {
-        const int slot = static_cast<int>(a.neighbour_slots[t]);
-        const float* frame = a.ring + static_cast<size_t>(slot) * a.frame_elems;
-        const uint32_t packed_t = t + 1;
-        float frame_d = kUnfilled;
-        uint32_t frame_pos = 0;
-        uint32_t sl[RECTS], sr[RECTS], st[RECTS], sb[RECTS];
-#pragma unroll
-        for (int i = 0; i < RECTS; ++i) {
-            sl[i] = 1;
-            sr[i] = 0;
-            st[i] = 1;
-            sb[i] = 0;
-        }
-#pragma unroll
-        for (int iy = 0; iy < COVERS; ++iy)
-#pragma unroll
-            for (int ix = 0; ix < COVERS; ++ix) {
-                const uint32_t bx = bx_lo + ix, by = by_lo + iy;
-                if (bx > bx_hi || by > by_hi) continue;
-                const uint32_t block = by * a.blocks_x + bx;
-                if (!(__ldg(a.confidence + t * a.conf_stride + block) >= a.c_min)) continue;
-                const int mvx = __ldg(a.mv_field + t * a.mv_stride + block * 2);
-                const int mvy = __ldg(a.mv_field + t * a.mv_stride + block * 2 + 1);
-                const uint32_t left = clamp_top_left(static_cast<int>(ax) + mvx - a.refine, max_x);
-                const uint32_t right = clamp_top_left(static_cast<int>(ax) + mvx + a.refine, max_x);
-                const uint32_t top = clamp_top_left(static_cast<int>(ay) + mvy - a.refine, max_y);
-                const uint32_t bottom = clamp_top_left(static_cast<int>(ay) + mvy + a.refine, max_y);
-                bool contained = false;
-#pragma unroll
-                for (int i = 0; i < RECTS; ++i)
-                    contained |= left >= sl[i] && right <= sr[i] && top >= st[i] && bottom <= sb[i];
-                if (!contained) {
-                    for (uint32_t cy = top; cy <= bottom; ++cy)
-                        for (uint32_t cx = left; cx <= right; ++cx) {
-                            const float d = reduce8(g, column_ssd<C>(anchor, frame, a.width, cx, cy, g.sub)) * scale;
-                            if (!(d < frame_d)) continue;
-                            bool skip = false;
-#pragma unroll
-                            for (int i = 0; i < RECTS; ++i)
-                                skip |= cy >= st[i] && cy <= sb[i] && cx >= sl[i] && cx <= sr[i];
-                            const uint32_t packed = pack_pos_t(cx, cy, packed_t);
-#pragma unroll
-                            for (int k = 0; k < FIRST; ++k) skip |= grid_pos[k] == packed;
-                            if (skip) continue;
-                            frame_d = d;
-                            frame_pos = packed;
-                        }
-                }
-                sl[iy * COVERS + ix] = left;
-                sr[iy * COVERS + ix] = right;
-                st[iy * COVERS + ix] = top;
-                sb[iy * COVERS + ix] = bottom;
-            }
-        float carry_d = frame_d;
-        uint32_t carry_pos = frame_pos;
-#pragma unroll
-        for (int j = 0; j < TAIL; ++j) {
-            const float held_d = grid_d[FIRST + j];
-            const uint32_t held_pos = grid_pos[FIRST + j];
-            if (carry_d < held_d) {
-                grid_d[FIRST + j] = carry_d;
-                grid_pos[FIRST + j] = carry_pos;
-                carry_d = held_d;
-                carry_pos = held_pos;
-            }
-        }
-    }
-}
-
-template <int C, int GF, int COVERS, int VOL = 0>
-__device__ __forceinline__ void search_volumes(const GroupCtx& g, const CollabLaunch& a, const uint32_t (&member_pos)[MAX_K],
-                                               float scale, float (&grid_d)[MAX_K], uint32_t (&grid_pos)[MAX_K]) {
-    if constexpr (VOL < MAX_K / GF) {
-        constexpr int FIRST = VOL * GF;
-        const uint32_t anchor_packed = member_pos[VOL];
-        const uint32_t ax = anchor_packed & 0x1FFFu, ay = (anchor_packed >> 13) & 0x1FFFu;
-        grid_pos[FIRST] = anchor_packed;
-        grid_d[FIRST] = 0.0f;
-#pragma unroll
-        for (int j = 1; j < GF; ++j) {
-            grid_pos[FIRST + j] = 0;
-            grid_d[FIRST + j] = kUnfilled;
-        }
-        float anchor[P * C];
-        const float* centre = a.ring + static_cast<size_t>(a.centre_slot) * a.frame_elems;
-#pragma unroll
-        for (int r = 0; r < P; ++r)
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                anchor[r * C + c] = __ldg(centre + ((static_cast<size_t>(ay) + r) * a.width + ax + g.sub) * C + c);
-        trajectory_search<C, GF, FIRST + 1, COVERS>(g, a, anchor, ax, ay, scale, grid_d, grid_pos);
-        search_volumes<C, GF, COVERS, VOL + 1>(g, a, member_pos, scale, grid_d, grid_pos);
-    }
-}
-
-// Keyed top-8 insert: the reference visits the window row by row and keeps ties in visiting order
-// (fused/plane_ops.rs:38-53), so its list is the 8 smallest (distance, visiting index) pairs. The
-// search here visits columns, comparing the pair, which keeps exactly the same list.
-__device__ __forceinline__ bool key_less(float d, uint32_t i, float bd, uint32_t bi) {
-    return d < bd || (d == bd && i < bi);
-}
-
-__device__ __forceinline__ void shift_insert8_key(const GroupCtx& g, float& best_d, uint32_t& best_i, float d,
-                                                  uint32_t i) {
-    const float prev_d = __shfl_up_sync(g.mask, best_d, 1, 8);
-    const uint32_t prev_i = __shfl_up_sync(g.mask, best_i, 1, 8);
-    if (key_less(d, i, best_d, best_i)) {
-        if (g.sub == 0 || !key_less(d, i, prev_d, prev_i)) {
-            best_d = d;
-            best_i = i;
-        } else {
-            best_d = prev_d;
-            best_i = prev_i;
-        }
-    }
-}
-
-template <int C>
-__device__ __forceinline__ void load_row(float (&dst)[C], const float* __restrict__ colp, uint32_t row, int width) {
-#pragma unroll
-    for (int c = 0; c < C; ++c) dst[c] = __ldg(colp + static_cast<size_t>(row) * width * C + c);
-}
-
-// The group sums of eight candidates at once, each lane's eight column distances in `v`: the same
-// pairwise tree as reduce8 (partners xor 1, then 2, then 4), each level keeping half the candidates
-// on each side, so every total has the bits reduce8 gives it. Lane `sub` ends with the total of
-// candidate (sub & 1) * 4 + (sub & 2) + ((sub >> 2) & 1).
-__device__ __forceinline__ float reduce_scatter8(const GroupCtx& g, const float (&v)[8]) {
-    const bool b0 = g.sub & 1, b1 = g.sub & 2, b2 = g.sub & 4;
-    float u[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float give = b0 ? v[j] : v[4 + j];
-        const float keep = b0 ? v[4 + j] : v[j];
-        u[j] = __fadd_rn(keep, __shfl_xor_sync(g.mask, give, 1));
-    }
-    float w[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const float give = b1 ? u[j] : u[2 + j];
-        const float keep = b1 ? u[2 + j] : u[j];
-        w[j] = __fadd_rn(keep, __shfl_xor_sync(g.mask, give, 2));
-    }
-    const float give = b2 ? w[0] : w[1];
-    const float keep = b2 ? w[1] : w[0];
-    return __fadd_rn(keep, __shfl_xor_sync(g.mask, give, 4));
-}
-
-__device__ __forceinline__ int scattered_candidate(int sub) { return (sub & 1) * 4 + (sub & 2) + ((sub >> 2) & 1); }
-
-// Eight candidate rows jb..jb+7 of window column `col` (the lane's sample column `colp`): `rows`
-// holds window rows jb..jb+6 on entry and jb+8..jb+14 on exit. Each candidate's distance is its
-// column sums in row order, the group's pairwise sum (reduce8's tree), times the channel scale;
-// the candidates that beat the list's worst key join it one at a time, in any order (the list is
-// the 8 smallest (distance, visiting index) pairs whatever the order they arrive in).
-template <int C>
-__device__ __forceinline__ void centre_batch(const GroupCtx& g, const float (&cur)[P * C], float (&rows)[15][C],
-                                             const float* __restrict__ colp, int width, uint32_t top, uint32_t jb,
-                                             uint32_t hh, uint32_t col, uint32_t ww, bool self_col,
-                                             uint32_t self_row, float scale, float& best_d, uint32_t& best_i,
-                                             float& worst_d, uint32_t& worst_i) {
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        if (jb + x < hh) {
-            load_row<C>(rows[7 + x], colp, top + jb + 7 + x, width);
-        } else {
-#pragma unroll
-            for (int c = 0; c < C; ++c) rows[7 + x][c] = 0.0f;
-        }
-    }
-    float v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        float sum = 0.0f;
-#pragma unroll
-        for (int r = 0; r < P; ++r)
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const float d = cur[r * C + c] - rows[k + r][c];
-                sum = __fadd_rn(sum, __fmul_rn(d, d));
-            }
-        v[k] = sum;
-    }
-    const uint32_t j = jb + static_cast<uint32_t>(scattered_candidate(g.sub));
-    float d = reduce_scatter8(g, v) * scale;
-    if (self_col && j == self_row) d = kSelfPin;
-    const uint32_t i = j * ww + col;
-    const bool wins = j < hh && d < kUnfilled && key_less(d, i, worst_d, worst_i);
-    unsigned m = __ballot_sync(g.mask, wins) & g.mask;
-    while (m) {
-        const int src = __ffs(m) - 1;
-        m &= m - 1;
-        const float dd = __shfl_sync(g.mask, d, src);
-        const uint32_t ii = __shfl_sync(g.mask, i, src);
-        if (key_less(dd, ii, worst_d, worst_i)) {  // uniform: every lane holds the same words
-            shift_insert8_key(g, best_d, best_i, dd, ii);
-            worst_d = __shfl_sync(g.mask, best_d, 7, 8);
-            worst_i = __shfl_sync(g.mask, best_i, 7, 8);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 7; ++r)
-#pragma unroll
-        for (int c = 0; c < C; ++c) rows[r][c] = rows[8 + r][c];
-}
-
-// Member words per reference patch: 8 packed positions, then k_use | use_grid << 8.
-constexpr int kMemberWords = 9;
-
-template <int C, int GF, int COVERS>
-__global__ void __launch_bounds__(kThreads, C == 1 ? 5 : 4) collab_search_kernel(CollabLaunch a) {
-    const int lane = threadIdx.x & 31;
-    const int group = threadIdx.x >> 3;
-    GroupCtx g;
-    g.sub = threadIdx.x & 7;
-    g.mask = 0xFFu << (lane & ~7);
-
-    const uint32_t refs_x = (a.width - P + STEP - 1) / STEP + 1;
-    const uint32_t ix = blockIdx.x * kGroups + group;
-    if (ix >= refs_x) return;  // the group's 8 lanes leave together; no barrier spans groups
-    const uint32_t iy = blockIdx.y;
-    const uint32_t max_x = a.width - P, max_y = a.height - P;
-    const uint32_t rx = min(ix * STEP, max_x), ry = min(iy * STEP, max_y);
-    const float scale = C == 1 ? 3.0f : 1.5f;
-    const float* centre = a.ring + static_cast<size_t>(a.centre_slot) * a.frame_elems;
-
-    float cur[P * C];
-#pragma unroll
-    for (int r = 0; r < P; ++r)
-#pragma unroll
-        for (int c = 0; c < C; ++c) cur[r * C + c] = __ldg(centre + ((static_cast<size_t>(ry) + r) * a.width + rx + g.sub) * C + c);
-
-    // Centre search (fused/centre.rs:213-258) over the clipped window, column by column, eight
-    // candidate rows at a time with the column's rows in registers: one load per candidate and lane,
-    // one reduce-scatter of the group per eight candidates.
-    const uint32_t left = clamp_top_left(static_cast<int>(rx) - a.spatial_radius, max_x);
-    const uint32_t right = clamp_top_left(static_cast<int>(rx) + a.spatial_radius, max_x);
-    const uint32_t top = clamp_top_left(static_cast<int>(ry) - a.spatial_radius, max_y);
-    const uint32_t bottom = clamp_top_left(static_cast<int>(ry) + a.spatial_radius, max_y);
-    const uint32_t ww = right - left + 1, hh = bottom - top + 1;
-    float best_d = kUnfilled, worst_d = kUnfilled;
-    uint32_t best_i = 0xFFFFFFFFu, worst_i = 0xFFFFFFFFu;
-    for (uint32_t cx = left; cx <= right; ++cx) {
-        const float* colp = centre + static_cast<size_t>(cx + g.sub) * C;
-        const bool self_col = cx == rx;
-        const uint32_t col = cx - left, self_row = ry - top;
-        float rows[15][C];
-#pragma unroll
-        for (int r = 0; r < P - 1; ++r) load_row<C>(rows[r], colp, top + r, a.width);
-        for (uint32_t jb = 0; jb < hh; jb += 8)
-            centre_batch<C>(g, cur, rows, colp, a.width, top, jb, hh, col, ww, self_col, self_row, scale, best_d,
-                            best_i, worst_d, worst_i);
-    }
-    const uint32_t n_live = ww * hh;
-    int k_use = 1;
-    while (static_cast<uint32_t>(k_use * 2) <= n_live && k_use * 2 <= a.k_max) k_use *= 2;
-    uint32_t member_pos[MAX_K];
-#pragma unroll
-    for (int m = 0; m < MAX_K; ++m) {
-        const uint32_t i = __shfl_sync(g.mask, best_i, m, 8);
-        member_pos[m] = i == 0xFFFFFFFFu ? 0u : pack_pos_t(left + i % ww, top + i / ww, 0);
-    }
-
-    bool use_grid = false;
-    if constexpr (GF > 1) {
-        if (a.k_max == MAX_K) {
-            float grid_d[MAX_K];
-            uint32_t grid_pos[MAX_K];
-            search_volumes<C, GF, COVERS>(g, a, member_pos, scale, grid_d, grid_pos);
-            use_grid = k_use == MAX_K;
-#pragma unroll
-            for (int v = 0; v < MAX_K / GF; ++v) use_grid = use_grid && grid_d[v * GF + GF - 1] < kUnfilled;
-            if (use_grid) {
-#pragma unroll
-                for (int m = 0; m < MAX_K; ++m) member_pos[m] = grid_pos[m];
-                k_use = MAX_K;
-            }
-        }
-    }
-    uint32_t* words = a.members + static_cast<size_t>(iy * refs_x + ix) * kMemberWords;
-    uint32_t mine = member_pos[0];
-#pragma unroll
-    for (int m = 1; m < MAX_K; ++m) mine = g.sub == m ? member_pos[m] : mine;
-    words[g.sub] = mine;
-    if (g.sub == 0) words[MAX_K] = static_cast<uint32_t>(k_use) | (use_grid ? 0x100u : 0u);
 }
 
 // What filter_group (fused/mod.rs:559-850) settles before its transforms: the members and their
@@ -1046,25 +687,15 @@ __global__ void __launch_bounds__(kThreads, 2) collab_adjoint_kernel(CollabLaunc
     }
 }
 
-template <int C, int GF, int COVERS>
-cudaError_t launch_cgc(const CollabLaunch& a, cudaStream_t stream) {
+template <int C, int GF>
+cudaError_t launch_cg(const CollabLaunch& a, cudaStream_t stream) {
+    const cudaError_t e = launch_collab_search(a, stream);
+    if (e != cudaSuccess) return e;
     const uint32_t refs_x = (a.width - P + STEP - 1) / STEP + 1;
     const uint32_t refs_y = (a.height - P + STEP - 1) / STEP + 1;
     dim3 grid((refs_x + kGroups - 1) / kGroups, refs_y);
-    collab_search_kernel<C, GF, COVERS><<<grid, kThreads, 0, stream>>>(a);
     collab_filter_kernel<C, GF><<<grid, kThreads, 0, stream>>>(a);
     return cudaGetLastError();
-}
-
-template <int C, int GF>
-cudaError_t launch_cg(const CollabLaunch& a, cudaStream_t stream) {
-    if (GF == 1) return launch_cgc<C, GF, 1>(a, stream);  // no volumes: the walk never runs
-    switch ((a.blksize + a.blk_step - 1) / a.blk_step) {
-        case 1: return launch_cgc<C, GF, 1>(a, stream);
-        case 2: return launch_cgc<C, GF, 2>(a, stream);
-        case 3: return launch_cgc<C, GF, 3>(a, stream);
-        default: return launch_cgc<C, GF, 4>(a, stream);
-    }
 }
 
 cudaError_t upload_taps() {

@@ -1,0 +1,774 @@
+// NL4D group search for sm_100a: the best 8 positions of the centre frame's spatial window for every
+// reference patch (fused/centre.rs:213-258), then the volumes along the neighbour frames' motion
+// (fused/trajectory.rs). Two launches per pass, joined by the member words.
+//
+// The centre search. The members are the 8 smallest (distance, visiting index) pairs, the distance
+// being an f32 sum in the restatement's own order, so those bits decide. Scoring all (2r+1)^2
+// candidates that way costs 192 unfused f32 operations each and bounded the pass (4K luma, r = 16:
+// 1,089 candidates, about 9 of the search's 14.0 ms; 1080p luma, r = 9: 0.97 of 1.70 ms). The scoring
+// below takes 2.67 and 0.44 ms, the search 7.3 and 1.17 ms (chroma of the 4K frame 4.24 -> 2.0 ms). But only a dozen candidates are ever near the best
+// eight, and telling the rest apart needs no exact bits. So the candidates are first scored on the
+// tensor cores: with samples c, n in units of codes around the middle code, exact in f16,
+//     sum c^2 - D = 2 sum c n - sum n^2
+// is a contraction over the 64 (128) samples of a patch whose f32 accumulation is the integer itself
+// or within a known bound of it. The larger of it ranks the smaller distance. Every thread keeps the
+// largest score of its own share of a patch's candidates (64 shares to a patch); the eighth largest of
+// those shares' maxima is reached by at least eight candidates, so a candidate whose score lies below
+// it by more than the error of both scores cannot be among the best eight. A second round of the same
+// products lists the candidates at or above that line, and the 8-lane group of the patch scores the
+// listed ones (nine or ten of 1,089 on noisy frames) in the exact order. A patch whose list overflows
+// (flat areas full of ties) and every patch of a tile whose samples overrun f16 goes through the exact
+// search of the whole window.
+//
+// The error of a score, in units of squared codes: the tensor core's accumulation (k16 steps of sums
+// below 3 * 64 C R^2, R the largest sample of the tile), the f32 distance's own rounding (1e-5 of it,
+// and the quotients' 2^-24 per sample), and, where the ring holds floats rather than codes, the samples'
+// rounding to f16: |sqrt(D) - sqrt(D~)| is at most the norm of the rounding of both patches.
+//
+// How. A CTA owns 8 x 4 reference patches (step 4), four groups of 8 (4 x 2) that share a staged tile of
+// 16-byte chunks, chunk (x, y) holding the eight samples x..x+7 of row y: patch row r of candidate
+// (x, y) is chunk (x, y + r), so ldmatrix gathers sixteen candidates' rows (the instruction's 16 rows)
+// straight from it, and the eight patches of a group (times 2, its 8 columns) stay in registers. Warps
+// take the window's rows in turn.
+
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <mutex>
+
+#include "collab_group.cuh"
+#include "kernels.h"
+
+namespace avd {
+
+namespace {
+
+using namespace collab_detail;
+
+// The lane's share of the distance from `ref` (its 8 x C column) to the candidate at (x, y).
+template <int C>
+__device__ __forceinline__ float column_ssd(const float (&ref)[P * C], const float* __restrict__ frame, int width,
+                                            uint32_t x, uint32_t y, int sub) {
+    float s = 0.0f;
+    const float* p = frame + (static_cast<size_t>(y) * width + x + sub) * C;
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            float d = ref[r * C + c] - __ldg(p + static_cast<size_t>(r) * width * C + c);
+            s = __fadd_rn(s, __fmul_rn(d, d));
+        }
+    }
+    return s;
+}
+
+__device__ __forceinline__ uint32_t covering_lo(uint32_t patch_start, uint32_t blksize, uint32_t step) {
+    const uint32_t overhang = max(patch_start + P, blksize) - blksize;
+    return (overhang + step - 1) / step;
+}
+
+// fused/trajectory.rs (clipped walk): for each neighbour frame the best candidate over one refine
+// rectangle per covering motion block (blocks under c_min skipped, rectangles already searched and
+// positions the group holds skipped), inserted into the volume's sorted tail. COVERS (the covering
+// blocks per axis, ceil(blksize / step)) is a template argument so the rectangles searched so far
+// stay in registers. A skipped candidate can only matter if it would beat the frame's best so far,
+// so the skip test runs for those alone; the winner is the same.
+template <int C, int GF, int FIRST, int COVERS>
+__device__ __forceinline__ void trajectory_search(const GroupCtx& g, const CollabLaunch& a, const float (&anchor)[P * C],
+                                                  uint32_t ax, uint32_t ay, float scale, float (&grid_d)[MAX_K],
+                                                  uint32_t (&grid_pos)[MAX_K]) {
+    constexpr int TAIL = GF - 1;
+    constexpr int RECTS = COVERS * COVERS;
+    const uint32_t max_x = a.width - P, max_y = a.height - P;
+    const uint32_t bx_hi = min(ax / a.blk_step, static_cast<uint32_t>(a.blocks_x - 1));
+    const uint32_t by_hi = min(ay / a.blk_step, static_cast<uint32_t>(a.blocks_y - 1));
+    const uint32_t bx_lo = min(covering_lo(ax, a.blksize, a.blk_step), bx_hi);
+    const uint32_t by_lo = min(covering_lo(ay, a.blksize, a.blk_step), by_hi);
+    for (int t = 0; t < 2 * a.radius; ++t) {
+        const int slot = static_cast<int>(a.neighbour_slots[t]);
+        const float* frame = a.ring + static_cast<size_t>(slot) * a.frame_elems;
+        const uint32_t packed_t = t + 1;
+        float frame_d = kUnfilled;
+        uint32_t frame_pos = 0;
+        uint32_t sl[RECTS], sr[RECTS], st[RECTS], sb[RECTS];
+#pragma unroll
+        for (int i = 0; i < RECTS; ++i) {
+            sl[i] = 1;
+            sr[i] = 0;
+            st[i] = 1;
+            sb[i] = 0;
+        }
+#pragma unroll
+        for (int iy = 0; iy < COVERS; ++iy)
+#pragma unroll
+            for (int ix = 0; ix < COVERS; ++ix) {
+                const uint32_t bx = bx_lo + ix, by = by_lo + iy;
+                if (bx > bx_hi || by > by_hi) continue;
+                const uint32_t block = by * a.blocks_x + bx;
+                if (!(__ldg(a.confidence + t * a.conf_stride + block) >= a.c_min)) continue;
+                const int mvx = __ldg(a.mv_field + t * a.mv_stride + block * 2);
+                const int mvy = __ldg(a.mv_field + t * a.mv_stride + block * 2 + 1);
+                const uint32_t left = clamp_top_left(static_cast<int>(ax) + mvx - a.refine, max_x);
+                const uint32_t right = clamp_top_left(static_cast<int>(ax) + mvx + a.refine, max_x);
+                const uint32_t top = clamp_top_left(static_cast<int>(ay) + mvy - a.refine, max_y);
+                const uint32_t bottom = clamp_top_left(static_cast<int>(ay) + mvy + a.refine, max_y);
+                bool contained = false;
+#pragma unroll
+                for (int i = 0; i < RECTS; ++i)
+                    contained |= left >= sl[i] && right <= sr[i] && top >= st[i] && bottom <= sb[i];
+                if (!contained) {
+                    for (uint32_t cy = top; cy <= bottom; ++cy)
+                        for (uint32_t cx = left; cx <= right; ++cx) {
+                            const float d = reduce8(g, column_ssd<C>(anchor, frame, a.width, cx, cy, g.sub)) * scale;
+                            if (!(d < frame_d)) continue;
+                            bool skip = false;
+#pragma unroll
+                            for (int i = 0; i < RECTS; ++i)
+                                skip |= cy >= st[i] && cy <= sb[i] && cx >= sl[i] && cx <= sr[i];
+                            const uint32_t packed = pack_pos_t(cx, cy, packed_t);
+#pragma unroll
+                            for (int k = 0; k < FIRST; ++k) skip |= grid_pos[k] == packed;
+                            if (skip) continue;
+                            frame_d = d;
+                            frame_pos = packed;
+                        }
+                }
+                sl[iy * COVERS + ix] = left;
+                sr[iy * COVERS + ix] = right;
+                st[iy * COVERS + ix] = top;
+                sb[iy * COVERS + ix] = bottom;
+            }
+        float carry_d = frame_d;
+        uint32_t carry_pos = frame_pos;
+#pragma unroll
+        for (int j = 0; j < TAIL; ++j) {
+            const float held_d = grid_d[FIRST + j];
+            const uint32_t held_pos = grid_pos[FIRST + j];
+            if (carry_d < held_d) {
+                grid_d[FIRST + j] = carry_d;
+                grid_pos[FIRST + j] = carry_pos;
+                carry_d = held_d;
+                carry_pos = held_pos;
+            }
+        }
+    }
+}
+
+template <int C, int GF, int COVERS, int VOL = 0>
+__device__ __forceinline__ void search_volumes(const GroupCtx& g, const CollabLaunch& a, const uint32_t (&member_pos)[MAX_K],
+                                               float scale, float (&grid_d)[MAX_K], uint32_t (&grid_pos)[MAX_K]) {
+    if constexpr (VOL < MAX_K / GF) {
+        constexpr int FIRST = VOL * GF;
+        const uint32_t anchor_packed = member_pos[VOL];
+        const uint32_t ax = anchor_packed & 0x1FFFu, ay = (anchor_packed >> 13) & 0x1FFFu;
+        grid_pos[FIRST] = anchor_packed;
+        grid_d[FIRST] = 0.0f;
+#pragma unroll
+        for (int j = 1; j < GF; ++j) {
+            grid_pos[FIRST + j] = 0;
+            grid_d[FIRST + j] = kUnfilled;
+        }
+        float anchor[P * C];
+        const float* centre = a.ring + static_cast<size_t>(a.centre_slot) * a.frame_elems;
+#pragma unroll
+        for (int r = 0; r < P; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+                anchor[r * C + c] = __ldg(centre + ((static_cast<size_t>(ay) + r) * a.width + ax + g.sub) * C + c);
+        trajectory_search<C, GF, FIRST + 1, COVERS>(g, a, anchor, ax, ay, scale, grid_d, grid_pos);
+        search_volumes<C, GF, COVERS, VOL + 1>(g, a, member_pos, scale, grid_d, grid_pos);
+    }
+}
+
+// Keyed top-8 insert: the reference visits the window row by row and keeps ties in visiting order
+// (fused/plane_ops.rs:38-53), so its list is the 8 smallest (distance, visiting index) pairs. The
+// search here visits columns, comparing the pair, which keeps exactly the same list.
+__device__ __forceinline__ bool key_less(float d, uint32_t i, float bd, uint32_t bi) {
+    return d < bd || (d == bd && i < bi);
+}
+
+__device__ __forceinline__ void shift_insert8_key(const GroupCtx& g, float& best_d, uint32_t& best_i, float d,
+                                                  uint32_t i) {
+    const float prev_d = __shfl_up_sync(g.mask, best_d, 1, 8);
+    const uint32_t prev_i = __shfl_up_sync(g.mask, best_i, 1, 8);
+    if (key_less(d, i, best_d, best_i)) {
+        if (g.sub == 0 || !key_less(d, i, prev_d, prev_i)) {
+            best_d = d;
+            best_i = i;
+        } else {
+            best_d = prev_d;
+            best_i = prev_i;
+        }
+    }
+}
+
+template <int C>
+__device__ __forceinline__ void load_row(float (&dst)[C], const float* __restrict__ colp, uint32_t row, int width) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) dst[c] = __ldg(colp + static_cast<size_t>(row) * width * C + c);
+}
+
+// The group sums of eight candidates at once, each lane's eight column distances in `v`: the same
+// pairwise tree as reduce8 (partners xor 1, then 2, then 4), each level keeping half the candidates
+// on each side, so every total has the bits reduce8 gives it. Lane `sub` ends with the total of
+// candidate (sub & 1) * 4 + (sub & 2) + ((sub >> 2) & 1).
+__device__ __forceinline__ float reduce_scatter8(const GroupCtx& g, const float (&v)[8]) {
+    const bool b0 = g.sub & 1, b1 = g.sub & 2, b2 = g.sub & 4;
+    float u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float give = b0 ? v[j] : v[4 + j];
+        const float keep = b0 ? v[4 + j] : v[j];
+        u[j] = __fadd_rn(keep, __shfl_xor_sync(g.mask, give, 1));
+    }
+    float w[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float give = b1 ? u[j] : u[2 + j];
+        const float keep = b1 ? u[2 + j] : u[j];
+        w[j] = __fadd_rn(keep, __shfl_xor_sync(g.mask, give, 2));
+    }
+    const float give = b2 ? w[0] : w[1];
+    const float keep = b2 ? w[1] : w[0];
+    return __fadd_rn(keep, __shfl_xor_sync(g.mask, give, 4));
+}
+
+__device__ __forceinline__ int scattered_candidate(int sub) { return (sub & 1) * 4 + (sub & 2) + ((sub >> 2) & 1); }
+
+// Eight candidate rows jb..jb+7 of window column `col` (the lane's sample column `colp`): `rows`
+// holds window rows jb..jb+6 on entry and jb+8..jb+14 on exit. Each candidate's distance is its
+// column sums in row order, the group's pairwise sum (reduce8's tree), times the channel scale;
+// the candidates that beat the list's worst key join it one at a time, in any order (the list is
+// the 8 smallest (distance, visiting index) pairs whatever the order they arrive in).
+template <int C>
+__device__ __forceinline__ void centre_batch(const GroupCtx& g, const float (&cur)[P * C], float (&rows)[15][C],
+                                             const float* __restrict__ colp, int width, uint32_t top, uint32_t jb,
+                                             uint32_t hh, uint32_t col, uint32_t ww, bool self_col,
+                                             uint32_t self_row, float scale, float& best_d, uint32_t& best_i,
+                                             float& worst_d, uint32_t& worst_i) {
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        if (jb + x < hh) {
+            load_row<C>(rows[7 + x], colp, top + jb + 7 + x, width);
+        } else {
+#pragma unroll
+            for (int c = 0; c < C; ++c) rows[7 + x][c] = 0.0f;
+        }
+    }
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int r = 0; r < P; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float d = cur[r * C + c] - rows[k + r][c];
+                sum = __fadd_rn(sum, __fmul_rn(d, d));
+            }
+        v[k] = sum;
+    }
+    const uint32_t j = jb + static_cast<uint32_t>(scattered_candidate(g.sub));
+    float d = reduce_scatter8(g, v) * scale;
+    if (self_col && j == self_row) d = kSelfPin;
+    const uint32_t i = j * ww + col;
+    const bool wins = j < hh && d < kUnfilled && key_less(d, i, worst_d, worst_i);
+    unsigned m = __ballot_sync(g.mask, wins) & g.mask;
+    while (m) {
+        const int src = __ffs(m) - 1;
+        m &= m - 1;
+        const float dd = __shfl_sync(g.mask, d, src);
+        const uint32_t ii = __shfl_sync(g.mask, i, src);
+        if (key_less(dd, ii, worst_d, worst_i)) {  // uniform: every lane holds the same words
+            shift_insert8_key(g, best_d, best_i, dd, ii);
+            worst_d = __shfl_sync(g.mask, best_d, 7, 8);
+            worst_i = __shfl_sync(g.mask, best_i, 7, 8);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 7; ++r)
+#pragma unroll
+        for (int c = 0; c < C; ++c) rows[r][c] = rows[8 + r][c];
+}
+
+
+// Every candidate of the clipped window in the exact order (fused/centre.rs:213-258), column by column,
+// eight candidate rows at a time with the column's rows in registers: one load per candidate and lane,
+// one reduce-scatter of the group per eight candidates.
+template <int C>
+__device__ __noinline__ void centre_full(const GroupCtx& g, const float (&cur)[P * C], const float* __restrict__ centre,
+                                         int width, uint32_t rx, uint32_t ry, uint32_t left, uint32_t right,
+                                         uint32_t top, uint32_t bottom, float scale, float& best_d, uint32_t& best_i) {
+    const uint32_t ww = right - left + 1, hh = bottom - top + 1;
+    float worst_d = kUnfilled;
+    uint32_t worst_i = 0xFFFFFFFFu;
+    for (uint32_t cx = left; cx <= right; ++cx) {
+        const float* colp = centre + static_cast<size_t>(cx + g.sub) * C;
+        const bool self_col = cx == rx;
+        const uint32_t col = cx - left, self_row = ry - top;
+        float rows[15][C];
+#pragma unroll
+        for (int r = 0; r < P - 1; ++r) load_row<C>(rows[r], colp, top + r, width);
+        for (uint32_t jb = 0; jb < hh; jb += 8)
+            centre_batch<C>(g, cur, rows, colp, width, top, jb, hh, col, ww, self_col, self_row, scale, best_d,
+                            best_i, worst_d, worst_i);
+    }
+}
+
+// The patch's members and group size from the group's list, into the member words.
+__device__ __forceinline__ void write_members(const GroupCtx& g, uint32_t* words, uint32_t best_i, uint32_t left,
+                                              uint32_t top, uint32_t ww, uint32_t hh, int k_max) {
+    const uint32_t n_live = ww * hh;
+    int k_use = 1;
+    while (static_cast<uint32_t>(k_use * 2) <= n_live && k_use * 2 <= k_max) k_use *= 2;
+    words[g.sub] = best_i == 0xFFFFFFFFu ? 0u : pack_pos_t(left + best_i % ww, top + best_i / ww, 0);
+    if (g.sub == 0) words[MAX_K] = static_cast<uint32_t>(k_use);
+}
+
+constexpr int kRefsX = 8, kRefsY = 4, kRefs = kRefsX * kRefsY;  // reference patches of one CTA
+constexpr int kWarps = 8, kScreenThreads = 32 * kWarps;         // one 8-lane group per patch
+constexpr int kList = 48;                                       // candidates listed per patch
+constexpr int kShares = kWarps * 8;                             // shares of a patch's candidates
+constexpr int kMaxRadius = 16;
+constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
+constexpr float kOutside = -1e30f;
+
+// Tile sizes for spatial radius r: candidate columns (whole 16s), candidate rows, staged rows.
+__host__ __device__ inline int screen_tiles(int r) { return (4 * (kRefsX - 1) + 1 + 2 * r + 15) / 16; }
+__host__ __device__ inline int screen_pitch(int r) { return 16 * screen_tiles(r) + 1; }
+__host__ __device__ inline int screen_rows(int r) { return 4 * (kRefsY - 1) + 1 + 2 * r; }
+
+template <int C>
+__host__ __device__ inline size_t screen_smem(int r) {
+    const size_t rows = screen_rows(r) + 7, cp = screen_pitch(r);
+    const size_t shares = static_cast<size_t>(kRefs) * kShares, sums = rows * cp;
+    return 16 * C * rows * cp + sizeof(float) * (sums > shares ? sums : shares) +
+           sizeof(float) * screen_rows(r) * cp + sizeof(float) * kRefs + sizeof(int) * kRefs +
+           sizeof(uint16_t) * kRefs * kList;
+}
+
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0,
+                                        float c1, float c2, float c3) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+
+extern __shared__ __align__(16) unsigned char screen_raw[];
+
+// One round over the CTA's candidates: `visit(nt, e, cell, score)` for every candidate inside the window
+// of patch e of group nt held by this thread (cell = row * 64 + column of the tile).
+template <int C, class Visit>
+__device__ __forceinline__ void score_round(const CollabLaunch& a, uint32_t chunk_addr, const float* __restrict__ sums,
+                                            int tiles, int cp, int rows_staged, const uint32_t (&b)[4][8 * C],
+                                            const int (&px)[4][2], const int (&py)[4], const int (&first_x)[2],
+                                            const int (&last_x)[2], const int (&first_y)[2], const int (&last_y)[2],
+                                            Visit visit) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2;
+    const int r2 = 2 * a.spatial_radius;
+    const int crows = screen_rows(a.spatial_radius);
+    // This lane's row of the instruction's matrices: matrix l / 8 is (row half, patch row of the pair).
+    const int half = (lane >> 3) & 1, k_sel = lane >> 4;
+    const uint32_t base = chunk_addr + 16u * static_cast<uint32_t>(k_sel * cp + (lane & 7) + 8 * half);
+    for (int cr = warp; cr < crows; cr += kWarps) {
+        for (int ct = 0; ct < tiles; ++ct) {
+            uint32_t m[4 * C][4];
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                    ldmatrix4(m[4 * c + ks], base + 16u * static_cast<uint32_t>((c * rows_staged + cr + 2 * ks) * cp + 16 * ct));
+            const int c0 = 16 * ct + g;
+            const float s0 = sums[cr * cp + c0], s1 = sums[cr * cp + c0 + 8];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int nx = nt & 1, ny = nt >> 1;
+                if (16 * ct + 15 < first_x[nx] || 16 * ct > last_x[nx] + r2 || cr < first_y[ny] || cr > last_y[ny] + r2)
+                    continue;
+                float d[4];
+                mma_f16(d, m[0], b[nt][0], b[nt][1], s0, s0, s1, s1);
+#pragma unroll
+                for (int ks = 1; ks < 4 * C; ++ks)
+                    mma_f16(d, m[ks], b[nt][2 * ks], b[nt][2 * ks + 1], d[0], d[1], d[2], d[3]);
+                const bool row_in = static_cast<unsigned>(cr - py[nt]) <= static_cast<unsigned>(r2);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const bool in0 = row_in && static_cast<unsigned>(c0 - px[nt][e]) <= static_cast<unsigned>(r2);
+                    const bool in1 = row_in && static_cast<unsigned>(c0 + 8 - px[nt][e]) <= static_cast<unsigned>(r2);
+                    visit(nt, e, cr * 64 + c0, in0 ? d[e] : kOutside, in1 ? d[2 + e] : kOutside);
+                }
+            }
+        }
+    }
+}
+
+template <int C>
+__global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_kernel(CollabLaunch a) {
+    const int R = a.spatial_radius;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gq = lane >> 2, t4 = lane & 3;
+    const int max_x = a.width - P, max_y = a.height - P;
+    const int refs_x = (a.width - P + STEP - 1) / STEP + 1, refs_y = (a.height - P + STEP - 1) / STEP + 1;
+    const int ix0 = blockIdx.x * kRefsX, iy0 = blockIdx.y * kRefsY;
+    const int ox = min(ix0 * STEP, max_x), oy = min(iy0 * STEP, max_y);  // the tile's first patch
+    const int tiles = screen_tiles(R), cp = screen_pitch(R), crows = screen_rows(R), rows = crows + 7;
+    const float* centre = a.ring + static_cast<size_t>(a.centre_slot) * a.frame_elems;
+
+    uint4* chunks = reinterpret_cast<uint4*>(screen_raw);  // [C][rows][cp]
+    float* squares = reinterpret_cast<float*>(chunks + C * rows * cp);  // row sums, then the shares' maxima
+    const int sq = max(rows * cp, kRefs * kShares);
+    float* sums = squares + sq;                      // [crows][cp]: minus the patch's sum of squares
+    float* line = sums + crows * cp;                 // [kRefs]: the score a listed candidate reaches
+    int* count = reinterpret_cast<int*>(line + kRefs);
+    uint16_t* list = reinterpret_cast<uint16_t*>(count + kRefs);
+
+    // ---- stage: 8 chunks of one row per task; consecutive lanes take consecutive rows, whose odd pitch
+    // spreads the 16-byte stores over the banks ----
+    const bool codes = a.ring_code_max > 0.0f && a.ring_code_max <= 4095.0f;
+    const float to_code = codes ? a.ring_code_max : 1023.0f;
+    const float mid = codes ? floorf(0.5f * a.ring_code_max + 0.5f) : 512.0f;
+    float worst = 0.0f;
+    bool bad = false;
+    const int segs = 2 * tiles;
+    for (int task = tid; task < rows * segs; task += kScreenThreads) {
+        const int seg = task / rows, y = task - seg * rows;
+        const int x0 = 8 * seg;
+        const int gy = min(max(oy - R + y, 0), a.height - 1);
+        const float* src = centre + static_cast<size_t>(gy) * a.width * C;
+        float part[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i] = 0.0f;
+        float v[C][16];
+#pragma unroll
+        for (int i = 0; i < 15; ++i) {
+            const int gx = min(max(ox - R + x0 + i, 0), a.width - 1);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float s = __ldg(src + static_cast<size_t>(gx) * C + c);
+                // codes: rounded to the code; floats: rounded to f16
+                const float x = codes ? fmaf(s, to_code, kRound - mid) - kRound
+                                      : __half2float(__float2half_rn(fmaf(s, to_code, -mid)));
+                bad |= !(fabsf(x) <= 2048.0f);
+                worst = fmaxf(worst, fabsf(x));
+                v[c][i] = x;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            v[c][15] = 0.0f;
+            float run = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 7; ++i) run = fmaf(v[c][i], v[c][i], run);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                run = fmaf(v[c][i + 7], v[c][i + 7], run);
+                part[i] += run;
+                run = fmaf(-v[c][i], v[c][i], run);
+            }
+            uint32_t even[8], odd[7];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const __half2 h = __floats2half2_rn(v[c][2 * i], v[c][2 * i + 1]);
+                even[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+#pragma unroll
+            for (int i = 0; i < 7; ++i) odd[i] = __funnelshift_r(even[i], even[i + 1], 16);
+            uint4* dst = chunks + (c * rows + y) * cp + x0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t* w = (i & 1) ? odd + i / 2 : even + i / 2;
+                dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) squares[y * cp + x0 + i] = part[i];
+    }
+    if (tid < kRefs) count[tid] = 0;
+    bad = __syncthreads_or(bad);
+    for (int task = tid; task < ((crows + 7) / 8) * 16 * tiles; task += kScreenThreads) {
+        const int run_y = task / (16 * tiles), x = task - run_y * 16 * tiles;
+        const int y0 = 8 * run_y;
+        const int gx = ox - R + x;
+        float run = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) run += squares[(y0 + i) * cp + x];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (y0 + i < crows) {
+                run += squares[(y0 + i + 7) * cp + x];
+                const int gy = oy - R + y0 + i;
+                const bool in = gx >= 0 && gx <= max_x && gy >= 0 && gy <= max_y;
+                sums[(y0 + i) * cp + x] = in ? -run : kOutside;
+                run -= squares[(y0 + i) * cp + x];
+            }
+        }
+    }
+    __syncthreads();
+
+    // The group's patch (column n of the instruction) and this thread's two (columns 2 t4, 2 t4 + 1), as
+    // positions in the tile: a patch's window starts at its own position less the tile's first patch.
+    const uint32_t chunk_addr = static_cast<uint32_t>(__cvta_generic_to_shared(chunks));
+    if (!bad) {
+        uint32_t b[4][8 * C];
+        int px[4][2], py[4], first_x[2], last_x[2], first_y[2], last_y[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            first_x[h] = min((ix0 + 4 * h) * STEP, max_x) - ox;
+            last_x[h] = min((ix0 + 4 * h + 3) * STEP, max_x) - ox;
+            first_y[h] = min((iy0 + 2 * h) * STEP, max_y) - oy;
+            last_y[h] = min((iy0 + 2 * h + 1) * STEP, max_y) - oy;
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+            const int nx = nt & 1, ny = nt >> 1;
+            const int qx = min((ix0 + 4 * nx + (gq & 3)) * STEP, max_x) - ox + R;
+            const int qy = min((iy0 + 2 * ny + (gq >> 2)) * STEP, max_y) - oy + R;
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const uint32_t word =
+                        reinterpret_cast<const uint32_t*>(chunks + (c * rows + qy + r) * cp + qx)[t4];
+                    const __half2 h = *reinterpret_cast<const __half2*>(&word);
+                    const __half2 h2x = __hadd2(h, h);
+                    b[nt][8 * c + r] = *reinterpret_cast<const uint32_t*>(&h2x);
+                }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) px[nt][e] = min((ix0 + 4 * nx + (2 * t4 & 3) + e) * STEP, max_x) - ox;
+            py[nt] = min((iy0 + 2 * ny + (t4 >> 1)) * STEP, max_y) - oy;
+        }
+
+        // ---- round 1: the largest score of every share ----
+        float top[4][2];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) top[nt][0] = top[nt][1] = kOutside;
+        score_round<C>(a, chunk_addr, sums, tiles, cp, rows, b, px, py, first_x, last_x, first_y, last_y,
+                       [&](int nt, int e, int, float s0, float s1) { top[nt][e] = fmaxf(top[nt][e], fmaxf(s0, s1)); });
+        __syncthreads();  // the row sums are no longer read; the shares take their place
+        float* shares = squares;
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int ref = (2 * (nt >> 1) + (t4 >> 1)) * kRefsX + 4 * (nt & 1) + (2 * t4 & 3) + e;
+                shares[ref * kShares + warp * 8 + gq] = top[nt][e];
+            }
+        // the tile's largest sample
+        __shared__ float worst_warp[kWarps];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+        if (lane == 0) worst_warp[warp] = worst;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) worst = fmaxf(worst, worst_warp[w]);
+        {
+            // The eighth largest share of the group's own patch, then the line.
+            const int ref = tid >> 3, sub = tid & 7;
+            const unsigned mask = 0xFFu << (lane & ~7);
+            float own[kShares / 8];
+#pragma unroll
+            for (int i = 0; i < kShares / 8; ++i) own[i] = shares[ref * kShares + sub * (kShares / 8) + i];
+            float eighth = kOutside;
+            for (int round = 0; round < 8; ++round) {
+                float m = own[0];
+#pragma unroll
+                for (int i = 1; i < kShares / 8; ++i) m = fmaxf(m, own[i]);
+                float all = m;
+                all = fmaxf(all, __shfl_xor_sync(mask, all, 1));
+                all = fmaxf(all, __shfl_xor_sync(mask, all, 2));
+                all = fmaxf(all, __shfl_xor_sync(mask, all, 4));
+                eighth = all;
+                const unsigned holders = __ballot_sync(mask, m == all) & mask;
+                if (lane == __ffs(holders) - 1) {
+                    bool taken = false;
+#pragma unroll
+                    for (int i = 0; i < kShares / 8; ++i) {
+                        const bool take = !taken && own[i] == all;
+                        taken |= take;
+                        if (take) own[i] = kOutside;
+                    }
+                }
+            }
+            if (sub == 0) {
+                const int qx = min((ix0 + ref % kRefsX) * STEP, max_x) - ox + R;
+                const int qy = min((iy0 + ref / kRefsX) * STEP, max_y) - oy + R;
+                const float n = 64.0f * C;
+                const float reach = 3.0f * n * worst * worst;  // no partial sum is larger
+                const float dist = fmaxf(-sums[qy * cp + qx] - eighth, 0.0f);
+                const float fixed = 4.0f + reach * (static_cast<float>(4 * C + 1) * 2.4e-7f);
+                const float dist1 = dist + fixed;
+                const float quotients = 4e-4f * sqrtf(n * dist1) + 1e-5f * dist1;
+                const float halves = codes ? 0.0f : 2.0f * sqrtf(n) * worst * 4.9e-4f;
+                const float slack = 2.0f * (fixed + quotients) + 4.0f * halves * (sqrtf(dist1) + halves);
+                line[ref] = fmaxf(eighth - slack, -1e29f);
+            }
+        }
+        __syncthreads();
+        // ---- round 2: list the candidates at or above the line ----
+        float bar[4][2];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                bar[nt][e] = line[(2 * (nt >> 1) + (t4 >> 1)) * kRefsX + 4 * (nt & 1) + (2 * t4 & 3) + e];
+        score_round<C>(a, chunk_addr, sums, tiles, cp, rows, b, px, py, first_x, last_x, first_y, last_y,
+                       [&](int nt, int e, int cell, float s0, float s1) {
+                           if (fmaxf(s0, s1) >= bar[nt][e]) {
+                               const int ref = (2 * (nt >> 1) + (t4 >> 1)) * kRefsX + 4 * (nt & 1) + (2 * t4 & 3) + e;
+                               if (s0 >= bar[nt][e]) {
+                                   const int at = atomicAdd(count + ref, 1);
+                                   if (at < kList) list[ref * kList + at] = static_cast<uint16_t>(cell);
+                               }
+                               if (s1 >= bar[nt][e]) {
+                                   const int at = atomicAdd(count + ref, 1);
+                                   if (at < kList) list[ref * kList + at] = static_cast<uint16_t>(cell + 8);
+                               }
+                           }
+                       });
+        __syncthreads();
+    }
+
+    // ---- the listed candidates in the exact order, one 8-lane group per patch ----
+    GroupCtx g;
+    g.sub = tid & 7;
+    g.mask = 0xFFu << (lane & ~7);
+    const int ref = tid >> 3;
+    const int ix = ix0 + ref % kRefsX, iy = iy0 + ref / kRefsX;
+    if (ix >= refs_x || iy >= refs_y) return;  // the group's 8 lanes leave together; no barrier follows
+    const uint32_t rx = min(ix * STEP, max_x), ry = min(iy * STEP, max_y);
+    const float scale = C == 1 ? 3.0f : 1.5f;
+    float cur[P * C];
+#pragma unroll
+    for (int r = 0; r < P; ++r)
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            cur[r * C + c] = __ldg(centre + ((static_cast<size_t>(ry) + r) * a.width + rx + g.sub) * C + c);
+    const uint32_t left = clamp_top_left(static_cast<int>(rx) - R, max_x);
+    const uint32_t right = clamp_top_left(static_cast<int>(rx) + R, max_x);
+    const uint32_t top_row = clamp_top_left(static_cast<int>(ry) - R, max_y);
+    const uint32_t bottom = clamp_top_left(static_cast<int>(ry) + R, max_y);
+    const uint32_t ww = right - left + 1, hh = bottom - top_row + 1;
+    float best_d = kUnfilled, worst_d = kUnfilled;
+    uint32_t best_i = 0xFFFFFFFFu, worst_i = 0xFFFFFFFFu;
+    const int listed = bad ? kList + 1 : count[ref];
+    if (listed > kList) {
+        centre_full<C>(g, cur, centre, a.width, rx, ry, left, right, top_row, bottom, scale, best_d, best_i);
+    } else {
+        for (int j0 = 0; j0 < listed; j0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int cell = list[ref * kList + min(j0 + k, listed - 1)];
+                v[k] = column_ssd<C>(cur, centre, a.width, ox - R + (cell & 63), oy - R + (cell >> 6), g.sub);
+            }
+            const int j = j0 + scattered_candidate(g.sub);
+            float d = reduce_scatter8(g, v) * scale;
+            const int cell = list[ref * kList + min(j, listed - 1)];
+            const uint32_t cx = ox - R + (cell & 63), cy = oy - R + (cell >> 6);
+            if (cx == rx && cy == ry) d = kSelfPin;
+            const uint32_t i = (cy - top_row) * ww + (cx - left);
+            const bool wins = j < listed && d < kUnfilled && key_less(d, i, worst_d, worst_i);
+            unsigned m = __ballot_sync(g.mask, wins) & g.mask;
+            while (m) {
+                const int src = __ffs(m) - 1;
+                m &= m - 1;
+                const float dd = __shfl_sync(g.mask, d, src);
+                const uint32_t ii = __shfl_sync(g.mask, i, src);
+                if (key_less(dd, ii, worst_d, worst_i)) {  // uniform: every lane holds the same words
+                    shift_insert8_key(g, best_d, best_i, dd, ii);
+                    worst_d = __shfl_sync(g.mask, best_d, 7, 8);
+                    worst_i = __shfl_sync(g.mask, best_i, 7, 8);
+                }
+            }
+        }
+    }
+    write_members(g, a.members + static_cast<size_t>(iy * refs_x + ix) * kMemberWords, best_i, left, top_row, ww, hh,
+                  a.k_max);
+}
+
+// The volumes: each anchor's walk through the neighbour frames; a full grid replaces the members.
+template <int C, int GF, int COVERS>
+__global__ void __launch_bounds__(kThreads, C == 1 ? 5 : 4) collab_walk_kernel(CollabLaunch a) {
+    const int lane = threadIdx.x & 31;
+    GroupCtx g;
+    g.sub = threadIdx.x & 7;
+    g.mask = 0xFFu << (lane & ~7);
+    const uint32_t refs_x = (a.width - P + STEP - 1) / STEP + 1;
+    const uint32_t ix = blockIdx.x * kGroups + (threadIdx.x >> 3);
+    if (ix >= refs_x) return;  // the group's 8 lanes leave together; no barrier spans groups
+    uint32_t* words = a.members + static_cast<size_t>(blockIdx.y * refs_x + ix) * kMemberWords;
+    const int k_use = static_cast<int>(words[MAX_K] & 0xFFu);
+    if (k_use != MAX_K) return;  // a smaller group keeps its members
+    uint32_t member_pos[MAX_K];
+#pragma unroll
+    for (int m = 0; m < MAX_K; ++m) member_pos[m] = words[m];
+    float grid_d[MAX_K];
+    uint32_t grid_pos[MAX_K];
+    search_volumes<C, GF, COVERS>(g, a, member_pos, C == 1 ? 3.0f : 1.5f, grid_d, grid_pos);
+    bool full = true;
+#pragma unroll
+    for (int v = 0; v < MAX_K / GF; ++v) full = full && grid_d[v * GF + GF - 1] < kUnfilled;
+    if (!full) return;
+    uint32_t mine = grid_pos[0];
+#pragma unroll
+    for (int m = 1; m < MAX_K; ++m) mine = g.sub == m ? grid_pos[m] : mine;
+    words[g.sub] = mine;
+    if (g.sub == 0) words[MAX_K] = static_cast<uint32_t>(MAX_K) | 0x100u;
+}
+
+template <int C>
+cudaError_t launch_centre(const CollabLaunch& a, cudaStream_t stream) {
+    const int refs_x = (a.width - P + STEP - 1) / STEP + 1, refs_y = (a.height - P + STEP - 1) / STEP + 1;
+    if (a.spatial_radius < 0 || a.spatial_radius > kMaxRadius) return cudaErrorInvalidValue;
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(collab_screen_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(screen_smem<C>(kMaxRadius)));
+    });
+    if (attr_err != cudaSuccess) return attr_err;
+    const dim3 grid((refs_x + kRefsX - 1) / kRefsX, (refs_y + kRefsY - 1) / kRefsY);
+    collab_screen_kernel<C><<<grid, kScreenThreads, screen_smem<C>(a.spatial_radius), stream>>>(a);
+    return cudaGetLastError();
+}
+
+template <int C, int GF, int COVERS>
+cudaError_t launch_walk(const CollabLaunch& a, cudaStream_t stream) {
+    const int refs_x = (a.width - P + STEP - 1) / STEP + 1, refs_y = (a.height - P + STEP - 1) / STEP + 1;
+    const dim3 grid((refs_x + kGroups - 1) / kGroups, refs_y);
+    collab_walk_kernel<C, GF, COVERS><<<grid, kThreads, 0, stream>>>(a);
+    return cudaGetLastError();
+}
+
+template <int C, int GF>
+cudaError_t launch_walk_covers(const CollabLaunch& a, cudaStream_t stream) {
+    switch ((a.blksize + a.blk_step - 1) / a.blk_step) {
+        case 1: return launch_walk<C, GF, 1>(a, stream);
+        case 2: return launch_walk<C, GF, 2>(a, stream);
+        case 3: return launch_walk<C, GF, 3>(a, stream);
+        default: return launch_walk<C, GF, 4>(a, stream);
+    }
+}
+
+template <int C>
+cudaError_t launch_c(const CollabLaunch& a, cudaStream_t stream) {
+    const cudaError_t e = launch_centre<C>(a, stream);
+    if (e != cudaSuccess || a.radius == 0 || a.k_max != MAX_K) return e;
+    return a.radius == 1 ? launch_walk_covers<C, 2>(a, stream) : launch_walk_covers<C, 4>(a, stream);
+}
+
+}  // namespace
+
+cudaError_t launch_collab_search(const CollabLaunch& a, cudaStream_t stream) {
+    return a.channels == 1 ? launch_c<1>(a, stream) : launch_c<2>(a, stream);
+}
+
+}  // namespace avd

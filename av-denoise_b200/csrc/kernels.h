@@ -147,8 +147,12 @@ struct CollabLaunch {
     // The empirical Wiener stage after the threshold (an extension the reference does not have):
     // each kept coefficient z of noise variance v scaled by z^2 / (z^2 + v).
     int wiener;
+    // The largest code of the integer format the ring was ingested from, or 0 where it holds any floats.
+    float ring_code_max;
 };
 
+// The group search of one pass into `members` (collab_search.cu), the first half of launch_collab.
+cudaError_t launch_collab_search(const CollabLaunch& args, cudaStream_t stream);
 cudaError_t launch_collab(const CollabLaunch& args, cudaStream_t stream);
 
 // The adjoint of one collab pass (collab.cu: collab_adjoint_kernel), run after the pass with the

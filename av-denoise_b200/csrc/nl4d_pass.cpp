@@ -834,6 +834,7 @@ class Nl4dPass final : public Pass {
         a.pool_ratio = pool_ratio_;
         a.pooled = opts_.pooled_threshold ? 1 : 0;
         a.wiener = opts_.wiener ? 1 : 0;
+        a.ring_code_max = in_.kind != AVD_SAMPLE_F32 ? sample_max_value(in_) : 0.0f;
         a.radius = static_cast<int>(d_);
         a.refine = static_cast<int>(opts_.refine);
         a.spatial_radius = static_cast<int>(opts_.spatial_radius);

@@ -117,3 +117,40 @@ def test_gpu_matches_oracle_on_random_passes(oracle, w, h, radius, sr, seed):
     assert np.array_equal(wsum, o_ws)
     assert np.array_equal(accum, o_acc)
     assert np.array_equal(gw.view(np.uint32), o_gw.view(np.uint32))
+
+
+def screen_frame(kind: str, w: int, h: int, c: int, rng) -> np.ndarray:
+    y, x = np.mgrid[0:h, 0:w].astype(np.float32)
+    base = 0.5 + 0.3 * np.sin(x * 0.21 + y * 0.13)[..., None] + rng.normal(0, 0.05, (h, w, c))
+    if kind == "flat":  # every candidate ties: the lists overflow
+        base = np.full((h, w, c), 0.25)
+        base[h // 2:, w // 2:] = 0.75
+    elif kind == "levels":  # four levels: many ties among the best eight
+        base = np.round(np.clip(base, 0, 1) * 3) / 3
+    elif kind == "wide":  # past the f16 range of the scores in places
+        base = base * 6 - 3
+        base[h // 3, w // 3] = 1e5
+    elif kind == "codes":
+        base = np.round(np.clip(base, 0, 1) * 255) / 255
+    return base.astype(np.float32)
+
+
+@pytest.mark.parametrize("kind,w,h,c,sr", [("noise", 8, 8, 1, 16), ("noise", 9, 10, 2, 3), ("noise", 75, 43, 1, 16),
+                                           ("codes", 61, 70, 2, 16), ("noise", 41, 25, 1, 1), ("flat", 64, 48, 1, 9),
+                                           ("levels", 66, 37, 1, 7), ("levels", 48, 48, 2, 12),
+                                           ("wide", 70, 52, 1, 9), ("wide", 40, 36, 2, 5)])
+def test_screened_search_picks_the_exact_members(oracle, kind, w, h, c, sr):
+    """The centre search scores candidates on the tensor cores and settles the best eight in the exact
+    order: tile and frame edges, one patch, lists that overflow and samples past f16, every accumulator
+    equal to the oracle's."""
+    rng = np.random.default_rng(w * h + c + sr)
+    ring = screen_frame(kind, w, h, c, rng)
+    case = dict(ring=ring.reshape(-1), width=w, height=h, channels=c, centre_slot=0, radius=0, spatial_radius=sr,
+                k_max=8, sigma=(0.03,) * c, lambda_ht=3.0, rho=0.0, kaiser_beta=2.0)
+    accum, wsum, gw = run_gpu(case)
+    kw = dict(case)
+    o_acc, o_ws, o_gw = oracle.collab_fused(kw.pop("ring"), kw.pop("width"), kw.pop("height"), kw.pop("channels"),
+                                            **kw)
+    assert np.array_equal(wsum, o_ws)
+    assert np.array_equal(accum, o_acc)
+    assert np.array_equal(gw.view(np.uint32), o_gw.view(np.uint32))

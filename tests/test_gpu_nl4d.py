@@ -63,6 +63,21 @@ def test_nl4d_luma_matches_oracle(oracle, w, h, n, d, sigma, sr):
     check(oracle, [[g[0]] for g in got], [[f[0]] for f in frames], fmt, d, sigma, spatial_radius=sr)
 
 
+@pytest.mark.parametrize("depth", [12, 16])
+def test_nl4d_deep_codes(oracle, depth):
+    """12-bit codes fill the f16 operands of the search's scores, 16-bit codes are rounded to them."""
+    w, h, d, sigma, sr = 68, 44, 1, 9.0 / 255, 8
+    fmt = avd.SampleFormat.u16(depth)
+    frames = clip(w, h, 4, depth=depth, seed=depth)
+    spec = avd.EngineSpec.nl4d(opts(d, sigma, spatial_radius=sr), None,
+                               avd.Geometry(w, h, avd.ChromaLayout.GRAY, fmt, fmt))
+    got = Runner(spec).run(frames)
+    want, _ = oracle_nl4d(oracle, [[f[0]] for f in frames], fmt, d, sigma, spatial_radius=sr)
+    assert len(got) == len(want)
+    for g, wn in zip(got, want):  # every sample: a tie band in codes would cover all of a 16-bit range
+        assert np.array_equal(g[0], wn[0])
+
+
 def test_nl4d_plain_threshold_10bit(oracle):
     w, h, d, sigma = 64, 48, 1, 8.0 / 255
     fmt = avd.SampleFormat.u16(10)
