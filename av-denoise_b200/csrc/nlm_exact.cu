@@ -31,8 +31,8 @@
 // the averaged samples are read from the window too), then every lane forms
 // distances two at a time as two independent chains (a pair's forward and backward offset, or two
 // spatial offsets), reading the centre patch as a broadcast and the taps at immediate offsets when
-// the patch radius is a template argument (0..3; a generic loop reading the frames covers larger
-// radii). The weights and the products I*w land in the warp's shared memory in offset order. The
+// the patch radius is a template argument (0..4, 4 being the default; a generic loop reading the
+// frames covers larger radii). The weights and the products I*w land in the warp's shared memory in offset order. The
 // passes are independent until they are added to the frame's accumulators, so the warp folds a
 // batch of passes at once: lane (pass, accumulator) walks its pass's offsets in order for one of
 // the C channel sums, the weight sum or the max weight; the pass results are then added to the
@@ -50,7 +50,7 @@ namespace avd {
 namespace {
 
 constexpr int kWarps = 4;               // 128 threads, one pixel per warp
-constexpr int kMaxTplS = 3;             // patch radii with a compile-time tap loop and staged windows
+constexpr int kMaxTplS = 4;             // patch radii with a compile-time tap loop and staged windows
 constexpr int kMaxItemFloats = 2048;    // per warp: the weights and products of one batch of passes
 
 __device__ __forceinline__ int clampc(int v, int limit) { return v < 0 ? 0 : (v >= limit ? limit - 1 : v); }
@@ -466,6 +466,7 @@ cudaError_t launch_c(const NlmLaunch& a, int sms, cudaStream_t stream) {
         case 1: return launch_cs<C, 1>(a, sms, stream);
         case 2: return launch_cs<C, 2>(a, sms, stream);
         case 3: return launch_cs<C, 3>(a, sms, stream);
+        case 4: return launch_cs<C, 4>(a, sms, stream);
         default: return launch_cs<C, -1>(a, sms, stream);
     }
 }
@@ -473,7 +474,7 @@ cudaError_t launch_c(const NlmLaunch& a, int sms, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t launch_nlm_exact(const NlmLaunch& a, cudaStream_t stream) {
-    static_assert(kMaxTplS == 3, "launch_c dispatches radii 0..3 to the staged kernel");
+    static_assert(kMaxTplS == 4, "launch_c dispatches radii 0..4 to the staged kernel");
     if (a.search_radius < 0 || a.search_radius > 8 || a.patch_radius < 0 || a.patch_radius > 16 || a.pairs < 0 ||
         a.pairs > kMaxPairs || (a.fix_list != nullptr) != (a.fix_count != nullptr))
         return cudaErrorInvalidValue;

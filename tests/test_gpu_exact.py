@@ -82,6 +82,8 @@ def run_exact(oracle, w, h, alg, chroma, d, a, s, strength, seed, **oracle_kw):
     (50, 31, 1, 3, 1, 10.0),
     (40, 24, 1, 2, 0, 20.0),
     (48, 32, 1, 3, 5, 30.0),
+    (53, 37, 2, 8, 4, 6.0),  # the default patch radius at the widest window
+    (41, 27, 0, 2, 4, 1.2),
     (40, 30, 0, 4, 9, 40.0),
     (6, 5, 1, 2, 1, 10.0),
 ])
