@@ -66,6 +66,7 @@ AvdStatus avd_batch_submit(const AvdBatchJob* jobs, size_t n_jobs, uint32_t chan
     bool fast = true;
     for (size_t j = 0; j < n_jobs; ++j) fast = fast && jobs[j].pair_offset == 0.0f && jobs[j].spatial_offset == 0.0f;
     int tiles = 0, max_pairs = 0;
+    bool shares = false;
     const float area = static_cast<float>((2 * patch_radius + 1) * (2 * patch_radius + 1));
     for (size_t j = 0; j < n_jobs; ++j) {
         const AvdBatchJob& b = jobs[j];
@@ -108,6 +109,8 @@ AvdStatus avd_batch_submit(const AvdBatchJob* jobs, size_t n_jobs, uint32_t chan
         a.wref = self_weight;
         a.fast = fast ? 1 : 0;
         a.out = reinterpret_cast<float*>(b.out);
+        a.variant = avd::cols_split(a);
+        shares = shares || a.variant > 1;
         max_pairs = std::max(max_pairs, d);
     }
     prefix[n_jobs] = tiles;
@@ -117,7 +120,7 @@ AvdStatus avd_batch_submit(const AvdBatchJob* jobs, size_t n_jobs, uint32_t chan
     e = avd::launch_nlm_batch(reinterpret_cast<const avd::NlmLaunch*>(dev_base + L.jobs),
                               reinterpret_cast<const int*>(dev_base + L.prefix), static_cast<int>(n_jobs),
                               reinterpret_cast<int*>(dev_base), static_cast<int>(channels),
-                              static_cast<int>(patch_radius), fast, static_cast<int>(search_radius), max_pairs, s);
+                              static_cast<int>(patch_radius), fast, static_cast<int>(search_radius), max_pairs, shares, s);
     if (e != cudaSuccess) return fail(AVD_ERR_GPU, std::string("batch launch: ") + cudaGetErrorString(e));
     // The staging copy above is pageable: cudaMemcpyAsync has consumed `host` before returning.
     return AVD_OK;

@@ -973,8 +973,9 @@ class NlmPass final : public Pass {
     // tune/driver: the window kernel's variant for this pass's shape, each timed once on this very
     // launch (without the exact-finish list) when the tuner has no choice for the shape yet.
     int tune_window(const NlmLaunch& a) {
+        // "nlm_window2": stores written before the column-pair tile hold choices among other variants.
         char key[160];
-        std::snprintf(key, sizeof(key), "nlm_window c%d s%d a%d d%d fast%d conf%d lut%d %dx%d", a.channels,
+        std::snprintf(key, sizeof(key), "nlm_window2 c%d s%d a%d d%d fast%d conf%d lut%d %dx%d", a.channels,
                       a.patch_radius, a.search_radius, a.pairs, a.fast, a.conf ? 1 : 0, a.spatial_lut ? 1 : 0,
                       a.width, a.height);
         const int variants = a.ref_ring ? 1 : nlm_window_variants(a.channels, a.patch_radius, a.fast != 0);

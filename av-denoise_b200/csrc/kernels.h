@@ -73,13 +73,25 @@ struct NlmLaunch {
     int* fix_list;
     int* fix_count;
     float code_max, fix_band;
-    // The window kernel's launch variant (0: the baseline), one of nlm_window_variants(): the same
-    // code built for a different number of resident CTAs per SM, so a variant trades registers for
-    // occupancy and changes how many waves a frame's tiles take, never the results.
+    // The window kernel's launch variant, one of nlm_window_variants(). Up to patch radius
+    // kColsMaxPatch: 0 the column-pair tile (nlm_cols.cuh), 1 the same with its tiles shared by twice as
+    // many CTAs, 2 the offset-pair tile (nlm_tile.cuh), the only one past that radius. Variants differ in
+    // the order of the sums over offsets, within the exact finish's band.
     int variant;
 };
 
 cudaError_t launch_nlm(const NlmLaunch& args, cudaStream_t stream);
+constexpr int kColsMaxPatch = 4;
+// The column-pair tile, `split` CTAs of a cluster to a tile, without (fast) and with noise offsets.
+cudaError_t launch_nlm_cols_fast(const NlmLaunch& args, int split, cudaStream_t stream);
+cudaError_t launch_nlm_cols_hq(const NlmLaunch& args, int split, cudaStream_t stream);
+cudaError_t launch_nlm_cols_batch_fast(const NlmLaunch* jobs, const int* prefix, int njobs, int* counter, int channels,
+                                       int patch_radius, int search_radius, bool shares, cudaStream_t stream);
+cudaError_t launch_nlm_cols_batch_hq(const NlmLaunch* jobs, const int* prefix, int njobs, int* counter, int channels,
+                                     int patch_radius, int search_radius, bool shares, cudaStream_t stream);
+// The CTAs a lone launch shares each tile by; a batch's jobs carry it in `variant` (`shares`: some job's
+// is above 1).
+int cols_split(const NlmLaunch& args);
 int nlm_window_variants(int channels, int patch_radius, bool fast);
 
 // The exact finish (nlm_exact.cu): every pixel of `args.fix_list[0 .. *args.fix_count)` (every pixel
@@ -113,7 +125,8 @@ cudaError_t launch_bilateral(const float* in, float* out, int width, int height,
 int nlm_tile_rows(int channels, int patch_radius);
 int nlm_tile_cols();
 cudaError_t launch_nlm_batch(const NlmLaunch* jobs, const int* prefix, int njobs, int* counter, int channels,
-                             int patch_radius, bool fast, int max_search_radius, int max_pairs, cudaStream_t stream);
+                             int patch_radius, bool fast, int max_search_radius, int max_pairs, bool shares,
+                             cudaStream_t stream);
 
 // One NL4D collaborative-filter pass (collab/kernels/fused/mod.rs:170): every reference patch of
 // the centre slot, scattered into the per-slot fixed-point accumulators.

@@ -48,32 +48,6 @@ __global__ void __launch_bounds__(kThreads, C == 1 && FAST ? 5 : 4) nlm_window_k
     nlm_tile<C, S, FAST>(a, blockIdx.x, blockIdx.y);
 }
 
-// The tuner's variants of the window kernel (patch radius up to kVariantMaxS): the same tile built
-// for MINB resident CTAs per SM. The baseline's MINB is 5 for luma without offsets and 4 otherwise;
-// variant 1 holds one CTA fewer (more registers), variant 2 one more.
-constexpr int kVariantMaxS = 4;
-template <int C, bool FAST>
-constexpr int baseline_minb() {
-    return C == 1 && FAST ? 5 : 4;
-}
-template <int C, int S, bool FAST, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) nlm_window_variant_kernel(NlmLaunch a) {
-    nlm_tile<C, S, FAST>(a, blockIdx.x, blockIdx.y);
-}
-
-template <int C, int S, bool FAST, int MINB>
-cudaError_t launch_variant(const NlmLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(nlm_window_variant_kernel<C, S, FAST, MINB>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    });
-    if (attr_err != cudaSuccess) return attr_err;
-    nlm_window_variant_kernel<C, S, FAST, MINB><<<grid, kThreads, smem, stream>>>(a);
-    return cudaGetLastError();
-}
-
 // Persistent batch: every CTA takes tiles from one counter until the batch's tiles run out. Tile t
 // belongs to the job j with prefix[j] <= t < prefix[j + 1]; jobs are whole launch descriptions.
 template <int C, int S, bool FAST>
@@ -113,11 +87,6 @@ cudaError_t launch_csf(const NlmLaunch& a, cudaStream_t stream) {
     if (attr_err != cudaSuccess) return attr_err;
     dim3 grid((a.width + kTX - 1) / kTX, (a.height + K::TY - 1) / K::TY);
     size_t smem = nlm_smem_bytes<C, S>(a.search_radius, a.pairs, false);
-    if constexpr (S <= kVariantMaxS) {
-        constexpr int base = baseline_minb<C, FAST>();
-        if (a.variant == 1) return launch_variant<C, S, FAST, base - 1>(a, grid, smem, stream);
-        if (a.variant == 2) return launch_variant<C, S, FAST, base + 1>(a, grid, smem, stream);
-    }
     nlm_window_kernel<C, S, FAST><<<grid, kThreads, smem, stream>>>(a);
     return cudaGetLastError();
 }
@@ -178,15 +147,35 @@ int nlm_tile_rows(int /*channels*/, int patch_radius) {
 int nlm_tile_cols() { return kTX; }
 
 int nlm_window_variants(int /*channels*/, int patch_radius, bool /*fast*/) {
-    return patch_radius <= kVariantMaxS ? 3 : 1;
+    return patch_radius <= kColsMaxPatch ? 3 : 1;
+}
+
+// How many CTAs of a cluster share a column-pair tile. A frame's tiles alone leave SMs idle below a few
+// CTAs each: from 3 to an SM on, one CTA per tile (957x539 chroma, 690 tiles: 121 us alone, 129 shared
+// by two); under that, the fewest that reach it, up to the 8 of a portable cluster (640x360, 300 tiles,
+// a = 7: 88 us alone, 69 by two, 80 by four; 203x117, 35 tiles, d = 1 a = 5: 118 alone, 70, 45, 35 by
+// eight), as long as each keeps about two window rows of work for the frames it stages.
+int cols_split(const NlmLaunch& a) {
+    const int tiles = ((a.width + kTX - 1) / kTX) * ((a.height + nlm_tile_rows(a.channels, a.patch_radius) - 1) /
+                                                     nlm_tile_rows(a.channels, a.patch_radius));
+    const int rows = (2 * a.pairs + 1) * (2 * a.search_radius + 1);
+    int split = 1;
+    while (split < 8 && tiles * split < 3 * 148 && rows >= 4 * split) split *= 2;
+    return split;
 }
 
 cudaError_t launch_nlm_batch(const NlmLaunch* jobs, const int* prefix, int njobs, int* counter, int channels,
-                             int patch_radius, bool fast, int max_search_radius, int max_pairs, cudaStream_t stream) {
+                             int patch_radius, bool fast, int max_search_radius, int max_pairs, bool shares,
+                             cudaStream_t stream) {
+    if (patch_radius <= kColsMaxPatch && (channels == 1 || channels == 2))
+        return fast ? launch_nlm_cols_batch_fast(jobs, prefix, njobs, counter, channels, patch_radius,
+                                                 max_search_radius, shares, stream)
+                    : launch_nlm_cols_batch_hq(jobs, prefix, njobs, counter, channels, patch_radius, max_search_radius,
+                                               shares, stream);
     if (channels == 1)
-        return batch_s<1, 0>(patch_radius, fast, jobs, prefix, njobs, counter, max_search_radius, max_pairs, stream);
+        return batch_s<1, kColsMaxPatch + 1>(patch_radius, fast, jobs, prefix, njobs, counter, max_search_radius, max_pairs, stream);
     if (channels == 2)
-        return batch_s<2, 0>(patch_radius, fast, jobs, prefix, njobs, counter, max_search_radius, max_pairs, stream);
+        return batch_s<2, kColsMaxPatch + 1>(patch_radius, fast, jobs, prefix, njobs, counter, max_search_radius, max_pairs, stream);
     return cudaErrorInvalidValue;
 }
 
@@ -195,6 +184,14 @@ cudaError_t launch_nlm(const NlmLaunch& a, cudaStream_t stream) {
         a.patch_radius > 16)
         return cudaErrorInvalidValue;
     if (a.ref_ring) return launch_nlm_ref(a, stream);
+    if (a.patch_radius <= kColsMaxPatch && (a.channels == 1 || a.channels == 2) && a.variant != 2) {
+        const int split = cols_split(a);
+        // Variant 1: tiles shared by twice as many CTAs, which evens out the last wave of a long window
+        // (1279x719 d = 4 a = 4: 665 us with one CTA per tile, 605 with two).
+        const int rows = (2 * a.pairs + 1) * (2 * a.search_radius + 1);
+        const int use = a.variant == 1 && split < 8 && rows >= 2 * split ? 2 * split : split;
+        return a.fast ? launch_nlm_cols_fast(a, use, stream) : launch_nlm_cols_hq(a, use, stream);
+    }
     if (a.channels == 1) return dispatch_s<1, 0>(a, stream);
     if (a.channels == 2) return dispatch_s<2, 0>(a, stream);
     return cudaErrorInvalidValue;

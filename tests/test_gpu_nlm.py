@@ -68,6 +68,25 @@ def test_luma_parity(oracle, w, h, depth, d, a, s, strength):
     check_group(oracle, [[g[0]] for g in got], [[f[0]] for f in frames], fmt, d, a, s, strength)
 
 
+@pytest.mark.parametrize("w,h,d,a,s,strength", [
+    (33, 29, 1, 6, 0, 12.0),   # one column and one row past a tile, the wide pitch
+    (31, 25, 2, 1, 1, 8.0),    # less than a tile, tiles shared by a cluster
+    (16, 57, 0, 8, 2, 10.0),   # a pair's second half empty, the widest window
+    (65, 24, 3, 4, 3, 7.0),    # an exact tile row
+    (97, 49, 1, 2, 4, 1.2),    # the default radii and strength
+])
+def test_column_pair_tile_edges(oracle, w, h, d, a, s, strength):
+    """Luma and chroma at the tile's remainders, for every patch radius of the column-pair tile."""
+    fmt = avd.SampleFormat.u8()
+    frames = clip(w, h, 4, chroma="444", seed=w + h)
+    spec = avd.EngineSpec.nlmeans(nlm(d, a, s, strength), nlm(d, a, s, strength),
+                                  avd.Geometry(w, h, avd.ChromaLayout.YUV444, fmt, fmt))
+    got = Runner(spec, tuning=avd.TuningConfig(mode="off")).run(frames)
+    check_group(oracle, [[g[0]] for g in got], [[f[0]] for f in frames], fmt, d, a, s, strength)
+    check_group(oracle, [[g[1], g[2]] for g in got], [[f[1], f[2]] for f in frames], fmt, d, a, s, strength,
+                chroma=True)
+
+
 def test_chroma_only_with_luma_passthrough(oracle):
     w, h = 144, 100
     frames = clip(w, h, 4, chroma="420", seed=3)
