@@ -358,6 +358,41 @@ struct Blocked {
     static constexpr int kWindow = kStride * kRows;
 };
 
+// One work item: candidate row item / kGroups, kWide offsets of it, from the staged block and window.
+template <int BLK, int R>
+__device__ __forceinline__ void blocked_item(int item, const float* centre_tile, const float* window, float* sads) {
+    using B = Blocked<BLK, R>;
+    const int dy = item / B::kGroups, dx0 = (item % B::kGroups) * B::kWide;
+    float part[B::kWide];
+#pragma unroll
+    for (int k = 0; k < B::kWide; ++k) part[k] = 0.0f;
+    for (int iy = 0; iy < BLK; ++iy) {
+        const float* wrow = window + (iy + dy) * B::kStride + dx0;
+        // The block row in registers, four samples per shared load (rows start 16-byte aligned).
+        const float4* crow = reinterpret_cast<const float4*>(centre_tile + iy * BLK);
+        float c[BLK];
+#pragma unroll
+        for (int q = 0; q < BLK / 4; ++q) {
+            const float4 v = crow[q];
+            c[4 * q] = v.x;
+            c[4 * q + 1] = v.y;
+            c[4 * q + 2] = v.z;
+            c[4 * q + 3] = v.w;
+        }
+        float w[BLK + B::kWide - 1];
+#pragma unroll
+        for (int k = 0; k < BLK + B::kWide - 1; ++k) w[k] = wrow[k];
+#pragma unroll
+        for (int ix = 0; ix < BLK; ++ix) {
+#pragma unroll
+            for (int k = 0; k < B::kWide; ++k) part[k] = __fadd_rn(part[k], fabsf(__fsub_rn(c[ix], w[ix + k])));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < B::kWide; ++k)
+        if (dx0 + k < B::kSide) sads[dy * B::kSide + dx0 + k] = part[k];
+}
+
 template <int BLK, int R>
 __device__ __forceinline__ void blocked_window(const SearchLevel& L, int64_t centre_base, int64_t nbr_base, int ox,
                                                int oy, int cdx, int cdy, float* centre_tile, float* window,
@@ -375,37 +410,7 @@ __device__ __forceinline__ void blocked_window(const SearchLevel& L, int64_t cen
                               clamp_to(wx0 + wx, L.width)];
     }
     __syncwarp();
-    for (int item = lane; item < B::kItems; item += 32) {
-        const int dy = item / B::kGroups, dx0 = (item % B::kGroups) * B::kWide;
-        float part[B::kWide];
-#pragma unroll
-        for (int k = 0; k < B::kWide; ++k) part[k] = 0.0f;
-        for (int iy = 0; iy < BLK; ++iy) {
-            const float* wrow = window + (iy + dy) * B::kStride + dx0;
-            // The block row in registers, four samples per shared load (rows start 16-byte aligned).
-            const float4* crow = reinterpret_cast<const float4*>(centre_tile + iy * BLK);
-            float c[BLK];
-#pragma unroll
-            for (int q = 0; q < BLK / 4; ++q) {
-                const float4 v = crow[q];
-                c[4 * q] = v.x;
-                c[4 * q + 1] = v.y;
-                c[4 * q + 2] = v.z;
-                c[4 * q + 3] = v.w;
-            }
-            float w[BLK + B::kWide - 1];
-#pragma unroll
-            for (int k = 0; k < BLK + B::kWide - 1; ++k) w[k] = wrow[k];
-#pragma unroll
-            for (int ix = 0; ix < BLK; ++ix) {
-#pragma unroll
-                for (int k = 0; k < B::kWide; ++k) part[k] = __fadd_rn(part[k], fabsf(__fsub_rn(c[ix], w[ix + k])));
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < B::kWide; ++k)
-            if (dx0 + k < B::kSide) sads[dy * B::kSide + dx0 + k] = part[k];
-    }
+    for (int item = lane; item < B::kItems; item += 32) blocked_item<BLK, R>(item, centre_tile, window, sads);
     __syncwarp();
     unsigned long long key = ~0ull;
     for (int i = lane; i < B::kSide * B::kSide; i += 32) {
@@ -686,10 +691,53 @@ __global__ void __launch_bounds__(64) flag_kernel(EscalateArgs e) {
     e.state[kStateFlag * sec + slot] = (low || on_edge || closest > kNeighbourDisagreement) ? 1.0f : 0.0f;
 }
 
-// escalate.rs:400-640 (`mc_escalate_search`, `coarse_search`).
-template <int C>
-__global__ void __launch_bounds__(((2 * C + 1) * (2 * C + 1) + 31) / 32 * 32) escalate_kernel(EscalateArgs e) {
-    __shared__ WindowScratch<C> w;
+// One window of a block of compile-time size BLK by the whole CTA, the result at thread 0: work items of
+// one candidate row and three adjacent offsets, as Blocked has them, over the CTA's threads (radius 8:
+// 102 items on 128 threads, where one thread per candidate takes 320 and two shared loads per term: the
+// escalations of a 12-frame 1279x719 d = 4 stream 14.1 -> 6.2 ms).
+template <int BLK, int R>
+__device__ __forceinline__ WinBest window_best_blocked(const SearchLevel& L, int64_t centre_base, int64_t nbr_base,
+                                                       int ox, int oy, int cdx, int cdy, WindowScratch<R>& w) {
+    using B = Blocked<BLK, R>;
+    static_assert(B::kWindow <= (kMaxBlk + 2 * R) * (kMaxBlk + 2 * R), "the window scratch holds the blocked rows");
+    const int t = threadIdx.x;
+    for (int i = t; i < BLK * BLK; i += blockDim.x) {
+        const int py = i / BLK, px = i % BLK;
+        w.centre_tile[i] = L.pyramid[centre_base + static_cast<int64_t>(clamp_to(oy + py, L.height)) * L.width +
+                                     clamp_to(ox + px, L.width)];
+    }
+    const int wx0 = ox + cdx - R, wy0 = oy + cdy - R;
+    for (int i = t; i < B::kWindow; i += blockDim.x) {
+        const int wy = i / B::kStride, wx = i % B::kStride;
+        w.window[i] = L.pyramid[nbr_base + static_cast<int64_t>(clamp_to(wy0 + wy, L.height)) * L.width +
+                                clamp_to(wx0 + wx, L.width)];
+    }
+    __syncthreads();
+    for (int item = t; item < B::kItems; item += blockDim.x)
+        blocked_item<BLK, R>(item, w.centre_tile, w.window, w.sads);
+    __syncthreads();
+    window_argmin<R>(w.sads, w.warp_keys, &w.best_index);
+    WinBest r{cdx, cdy, kNoSad, 0.0f, 0.0f, cdx, cdy};
+    if (t == 0) r = window_result<R>(w.sads, w.best_index, cdx, cdy, false, false);
+    __syncthreads();  // thread 0 is done with the scores
+    return r;
+}
+
+// escalate.rs:400-640 (`mc_escalate_search`, `coarse_search`). BLK and CBLK: the block sizes of the two
+// levels where they are the usual 16 and 8 (the blocked windows), or 0 for any size.
+constexpr int kEscalateThreads = 128;
+template <int C, int BLK, int CBLK>
+__global__ void __launch_bounds__(BLK ? kEscalateThreads : ((2 * C + 1) * (2 * C + 1) + 31) / 32 * 32)
+    escalate_kernel(EscalateArgs e) {
+    __shared__ __align__(16) WindowScratch<C> w;
+    auto coarse_best = [&](int64_t cb, int64_t nb, int ox, int oy, int dx, int dy) {
+        if constexpr (CBLK != 0) return window_best_blocked<CBLK, C>(e.Lc, cb, nb, ox, oy, dx, dy, w);
+        else return window_best<C>(e.Lc, cb, nb, ox, oy, dx, dy, w, false, false);
+    };
+    auto fine_best = [&](int64_t cb, int64_t nb, int ox, int oy, int dx, int dy) {
+        if constexpr (BLK != 0) return window_best_blocked<BLK, C>(e.L, cb, nb, ox, oy, dx, dy, w);
+        else return window_best<C>(e.L, cb, nb, ox, oy, dx, dy, w, false, false);
+    };
     __shared__ int coarse_vec[2];
     const int bx = blockIdx.x, by = blockIdx.y, n = blockIdx.z;
     const int64_t sec = escalate_section(e);
@@ -707,10 +755,10 @@ __global__ void __launch_bounds__(((2 * C + 1) * (2 * C + 1) + 31) / 32 * 32) es
         const int64_t cb = e.Lc.level_base + static_cast<int64_t>(e.centre_slot) * e.Lc.slot_pixels;
         const int64_t nb = e.Lc.level_base + static_cast<int64_t>(nslot) * e.Lc.slot_pixels;
         const int ox = bx * e.L.step / e.scale, oy = by * e.L.step / e.scale;
-        WinBest cbest = window_best<C>(e.Lc, cb, nb, ox, oy, 0, 0, w, false, false);
+        WinBest cbest = coarse_best(cb, nb, ox, oy, 0, 0);
         int mdx, mdy;
         if (model_window(e.predictions, n, ox, oy, e.Lc.blksize, e.scale, e.Lc.width, e.Lc.height, C, 0, 0, &mdx, &mdy)) {
-            const WinBest ch = window_best<C>(e.Lc, cb, nb, ox, oy, mdx, mdy, w, false, false);
+            const WinBest ch = coarse_best(cb, nb, ox, oy, mdx, mdy);
             const float bias = __fmul_rn(__fmul_rn(kModelCandidateBias, sad_floor), e.floor_scale);
             if (threadIdx.x == 0 && __fadd_rn(ch.sad, bias) < cbest.sad) cbest = ch;
         }
@@ -724,9 +772,9 @@ __global__ void __launch_bounds__(((2 * C + 1) * (2 * C + 1) + 31) / 32 * 32) es
     }
     const int64_t cb = static_cast<int64_t>(e.centre_slot) * e.L.slot_pixels;
     const int64_t nb = static_cast<int64_t>(nslot) * e.L.slot_pixels;
-    WinBest best = window_best<C>(e.L, cb, nb, bx * e.L.step, by * e.L.step, cdx, cdy, w, false, false);
+    WinBest best = fine_best(cb, nb, bx * e.L.step, by * e.L.step, cdx, cdy);
     if (e.widen && (kx != cdx || ky != cdy)) {  // uniform: every thread holds the same vectors
-        const WinBest ch = window_best<C>(e.L, cb, nb, bx * e.L.step, by * e.L.step, kx, ky, w, false, false);
+        const WinBest ch = fine_best(cb, nb, bx * e.L.step, by * e.L.step, kx, ky);
         if (threadIdx.x == 0 && __fadd_rn(ch.sad, margin) < best.sad) best = ch;
     }
     if (threadIdx.x != 0) return;
@@ -744,7 +792,13 @@ template <int R>
 cudaError_t launch_escalate(int radius, const EscalateArgs& e, dim3 grid, cudaStream_t s) {
     if (radius == R) {
         constexpr int kCand = (2 * R + 1) * (2 * R + 1);
-        escalate_kernel<R><<<grid, ((kCand + 31) / 32) * 32, 0, s>>>(e);
+        if constexpr (R >= 4) {
+            if (e.L.blksize == 16 && (!e.widen || e.Lc.blksize == 8)) {
+                escalate_kernel<R, 16, 8><<<grid, kEscalateThreads, 0, s>>>(e);
+                return cudaGetLastError();
+            }
+        }
+        escalate_kernel<R, 0, 0><<<grid, ((kCand + 31) / 32) * 32, 0, s>>>(e);
         return cudaGetLastError();
     }
     if constexpr (R < kMaxRadius) {
