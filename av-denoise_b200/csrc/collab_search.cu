@@ -6,9 +6,9 @@
 // being an f32 sum in the restatement's own order, so those bits decide. Scoring all (2r+1)^2
 // candidates that way costs 192 unfused f32 operations each and bounded the pass (4K luma, r = 16:
 // 1,089 candidates, about 9 of the search's 14.0 ms; 1080p luma, r = 9: 0.97 of 1.70 ms). The scoring
-// below takes 2.67 and 0.44 ms, the search 7.3 and 1.17 ms (chroma of the 4K frame 4.24 -> 2.0 ms). But only a dozen candidates are ever near the best
-// eight, and telling the rest apart needs no exact bits. So the candidates are first scored on the
-// tensor cores: with samples c, n in units of codes around the middle code, exact in f16,
+// below takes 2.67 and 0.44 ms (chroma of the 4K frame 1.3). But only a dozen candidates are ever near
+// the best eight, and telling the rest apart needs no exact bits. So the candidates are first scored on
+// the tensor cores: with samples c, n in units of codes around the middle code, exact in f16,
 //     sum c^2 - D = 2 sum c n - sum n^2
 // is a contraction over the 64 (128) samples of a patch whose f32 accumulation is the integer itself
 // or within a known bound of it. The larger of it ranks the smaller distance. Every thread keeps the
@@ -66,119 +66,6 @@ __device__ __forceinline__ float column_ssd(const float (&ref)[P * C], const flo
 __device__ __forceinline__ uint32_t covering_lo(uint32_t patch_start, uint32_t blksize, uint32_t step) {
     const uint32_t overhang = max(patch_start + P, blksize) - blksize;
     return (overhang + step - 1) / step;
-}
-
-// fused/trajectory.rs (clipped walk): for each neighbour frame the best candidate over one refine
-// rectangle per covering motion block (blocks under c_min skipped, rectangles already searched and
-// positions the group holds skipped), inserted into the volume's sorted tail. COVERS (the covering
-// blocks per axis, ceil(blksize / step)) is a template argument so the rectangles searched so far
-// stay in registers. A skipped candidate can only matter if it would beat the frame's best so far,
-// so the skip test runs for those alone; the winner is the same.
-template <int C, int GF, int FIRST, int COVERS>
-__device__ __forceinline__ void trajectory_search(const GroupCtx& g, const CollabLaunch& a, const float (&anchor)[P * C],
-                                                  uint32_t ax, uint32_t ay, float scale, float (&grid_d)[MAX_K],
-                                                  uint32_t (&grid_pos)[MAX_K]) {
-    constexpr int TAIL = GF - 1;
-    constexpr int RECTS = COVERS * COVERS;
-    const uint32_t max_x = a.width - P, max_y = a.height - P;
-    const uint32_t bx_hi = min(ax / a.blk_step, static_cast<uint32_t>(a.blocks_x - 1));
-    const uint32_t by_hi = min(ay / a.blk_step, static_cast<uint32_t>(a.blocks_y - 1));
-    const uint32_t bx_lo = min(covering_lo(ax, a.blksize, a.blk_step), bx_hi);
-    const uint32_t by_lo = min(covering_lo(ay, a.blksize, a.blk_step), by_hi);
-    for (int t = 0; t < 2 * a.radius; ++t) {
-        const int slot = static_cast<int>(a.neighbour_slots[t]);
-        const float* frame = a.ring + static_cast<size_t>(slot) * a.frame_elems;
-        const uint32_t packed_t = t + 1;
-        float frame_d = kUnfilled;
-        uint32_t frame_pos = 0;
-        uint32_t sl[RECTS], sr[RECTS], st[RECTS], sb[RECTS];
-#pragma unroll
-        for (int i = 0; i < RECTS; ++i) {
-            sl[i] = 1;
-            sr[i] = 0;
-            st[i] = 1;
-            sb[i] = 0;
-        }
-#pragma unroll
-        for (int iy = 0; iy < COVERS; ++iy)
-#pragma unroll
-            for (int ix = 0; ix < COVERS; ++ix) {
-                const uint32_t bx = bx_lo + ix, by = by_lo + iy;
-                if (bx > bx_hi || by > by_hi) continue;
-                const uint32_t block = by * a.blocks_x + bx;
-                if (!(__ldg(a.confidence + t * a.conf_stride + block) >= a.c_min)) continue;
-                const int mvx = __ldg(a.mv_field + t * a.mv_stride + block * 2);
-                const int mvy = __ldg(a.mv_field + t * a.mv_stride + block * 2 + 1);
-                const uint32_t left = clamp_top_left(static_cast<int>(ax) + mvx - a.refine, max_x);
-                const uint32_t right = clamp_top_left(static_cast<int>(ax) + mvx + a.refine, max_x);
-                const uint32_t top = clamp_top_left(static_cast<int>(ay) + mvy - a.refine, max_y);
-                const uint32_t bottom = clamp_top_left(static_cast<int>(ay) + mvy + a.refine, max_y);
-                bool contained = false;
-#pragma unroll
-                for (int i = 0; i < RECTS; ++i)
-                    contained |= left >= sl[i] && right <= sr[i] && top >= st[i] && bottom <= sb[i];
-                if (!contained) {
-                    for (uint32_t cy = top; cy <= bottom; ++cy)
-                        for (uint32_t cx = left; cx <= right; ++cx) {
-                            const float d = reduce8(g, column_ssd<C>(anchor, frame, a.width, cx, cy, g.sub)) * scale;
-                            if (!(d < frame_d)) continue;
-                            bool skip = false;
-#pragma unroll
-                            for (int i = 0; i < RECTS; ++i)
-                                skip |= cy >= st[i] && cy <= sb[i] && cx >= sl[i] && cx <= sr[i];
-                            const uint32_t packed = pack_pos_t(cx, cy, packed_t);
-#pragma unroll
-                            for (int k = 0; k < FIRST; ++k) skip |= grid_pos[k] == packed;
-                            if (skip) continue;
-                            frame_d = d;
-                            frame_pos = packed;
-                        }
-                }
-                sl[iy * COVERS + ix] = left;
-                sr[iy * COVERS + ix] = right;
-                st[iy * COVERS + ix] = top;
-                sb[iy * COVERS + ix] = bottom;
-            }
-        float carry_d = frame_d;
-        uint32_t carry_pos = frame_pos;
-#pragma unroll
-        for (int j = 0; j < TAIL; ++j) {
-            const float held_d = grid_d[FIRST + j];
-            const uint32_t held_pos = grid_pos[FIRST + j];
-            if (carry_d < held_d) {
-                grid_d[FIRST + j] = carry_d;
-                grid_pos[FIRST + j] = carry_pos;
-                carry_d = held_d;
-                carry_pos = held_pos;
-            }
-        }
-    }
-}
-
-template <int C, int GF, int COVERS, int VOL = 0>
-__device__ __forceinline__ void search_volumes(const GroupCtx& g, const CollabLaunch& a, const uint32_t (&member_pos)[MAX_K],
-                                               float scale, float (&grid_d)[MAX_K], uint32_t (&grid_pos)[MAX_K]) {
-    if constexpr (VOL < MAX_K / GF) {
-        constexpr int FIRST = VOL * GF;
-        const uint32_t anchor_packed = member_pos[VOL];
-        const uint32_t ax = anchor_packed & 0x1FFFu, ay = (anchor_packed >> 13) & 0x1FFFu;
-        grid_pos[FIRST] = anchor_packed;
-        grid_d[FIRST] = 0.0f;
-#pragma unroll
-        for (int j = 1; j < GF; ++j) {
-            grid_pos[FIRST + j] = 0;
-            grid_d[FIRST + j] = kUnfilled;
-        }
-        float anchor[P * C];
-        const float* centre = a.ring + static_cast<size_t>(a.centre_slot) * a.frame_elems;
-#pragma unroll
-        for (int r = 0; r < P; ++r)
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                anchor[r * C + c] = __ldg(centre + ((static_cast<size_t>(ay) + r) * a.width + ax + g.sub) * C + c);
-        trajectory_search<C, GF, FIRST + 1, COVERS>(g, a, anchor, ax, ay, scale, grid_d, grid_pos);
-        search_volumes<C, GF, COVERS, VOL + 1>(g, a, member_pos, scale, grid_d, grid_pos);
-    }
 }
 
 // Keyed top-8 insert: the reference visits the window row by row and keeps ties in visiting order
@@ -694,33 +581,196 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
                   a.k_max);
 }
 
-// The volumes: each anchor's walk through the neighbour frames; a full grid replaces the members.
-template <int C, int GF, int COVERS>
-__global__ void __launch_bounds__(kThreads, C == 1 ? 5 : 4) collab_walk_kernel(CollabLaunch a) {
-    const int lane = threadIdx.x & 31;
+// One block of a refine rectangle: up to 5 x 5 candidates from (x0, y0), each scored in the exact order.
+// `minus` is the lane's anchor column negated. A lane reads a candidate column once for all its candidate
+// rows: 60 loads for 25 candidates, where one candidate at a time takes 200 and a group sum of its own
+// each. Candidate c of the block is column c / 5, row c % 5; lane `sub` ends with candidates
+// 8 b + scattered_candidate(sub), b = 0..2, and lane 0 with candidate 24, in d[b] (kUnfilled outside).
+constexpr int kBlk = 5;
+
+template <int C>
+__device__ __forceinline__ void score_block(const GroupCtx& g, const float (&minus)[P * C],
+                                            const float* __restrict__ frame, int width, uint32_t x0, uint32_t y0,
+                                            uint32_t right, uint32_t bottom, float scale, float (&d)[4]) {
+    float v[kBlk * kBlk];
+    const uint32_t last = bottom + P - 1;  // the last row any candidate reads
+#pragma unroll
+    for (int q = 0; q < kBlk; ++q) {
+        const float* p = frame + static_cast<size_t>(min(x0 + q, right) + g.sub) * C;
+        float rows[kBlk + P - 1][C];
+#pragma unroll
+        for (int r = 0; r < kBlk + P - 1; ++r) {
+            const size_t off = static_cast<size_t>(min(y0 + r, last)) * width * C;
+#pragma unroll
+            for (int c = 0; c < C; ++c) rows[r][c] = __ldg(p + off + c);
+        }
+#pragma unroll
+        for (int k = 0; k < kBlk; ++k) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int r = 0; r < P; ++r)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    // candidate - anchor: the negated difference has the same square
+                    const float diff = __fadd_rn(rows[k + r][c], minus[r * C + c]);
+                    sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+                }
+            v[kBlk * q + k] = sum;
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const int c = b < 3 ? 8 * b + scattered_candidate(g.sub) : 24;
+        float total;
+        if (b < 3) {
+            const float part[8] = {v[8 * (b % 3)], v[8 * (b % 3) + 1], v[8 * (b % 3) + 2], v[8 * (b % 3) + 3],
+                                   v[8 * (b % 3) + 4], v[8 * (b % 3) + 5], v[8 * (b % 3) + 6], v[8 * (b % 3) + 7]};
+            total = reduce_scatter8(g, part) * scale;
+        } else {
+            total = reduce8(g, v[24]) * scale;
+        }
+        const uint32_t cx = x0 + c / kBlk, cy = y0 + c % kBlk;
+        d[b] = cx <= right && cy <= bottom && (b < 3 || g.sub == 0) ? total : kUnfilled;
+    }
+}
+
+// The volumes (fused/trajectory.rs, clipped walk): each anchor's walk through the neighbour frames. Per
+// frame, the best candidate over one refine rectangle per covering motion block (blocks under c_min
+// skipped, rectangles already searched and positions the earlier volumes hold skipped) joins the
+// volume's sorted tail; a full grid replaces the members. The reference visits a rectangle row by row
+// and keeps the first of equal distances: the least (distance, visiting index) of the candidates not
+// skipped, taken if it beats the frame's best so far. Lane `sub` holds grid slot `sub`; the rectangles
+// searched so far and the held positions are in the group's shared memory, so the volumes, frames and
+// rectangles are loops around one copy of the scoring: 4.67 -> 3.97 ms per 4K luma pass (d = 3), 0.73 ->
+// 0.56 at 1080p (d = 2), against one candidate at a time in fully unrolled rectangles. The distances' 600
+// unfused f32 operations per rectangle and lane, which must keep their order, bound it; packed f32x2
+// takes the pipe as long. Four CTAs per SM: 3.97 ms, five (96 registers, spills) 4.32.
+constexpr int kMaxRects = 16;  // four covering blocks per axis
+
+template <int C>
+__global__ void __launch_bounds__(kThreads, 4) collab_walk_kernel(CollabLaunch a, int gf) {
+    __shared__ uint4 rects[kGroups][kMaxRects];
+    __shared__ uint32_t held[kGroups][MAX_K];
+    const int lane = threadIdx.x & 31, group = threadIdx.x >> 3;
     GroupCtx g;
     g.sub = threadIdx.x & 7;
     g.mask = 0xFFu << (lane & ~7);
     const uint32_t refs_x = (a.width - P + STEP - 1) / STEP + 1;
-    const uint32_t ix = blockIdx.x * kGroups + (threadIdx.x >> 3);
+    const uint32_t ix = blockIdx.x * kGroups + group;
     if (ix >= refs_x) return;  // the group's 8 lanes leave together; no barrier spans groups
     uint32_t* words = a.members + static_cast<size_t>(blockIdx.y * refs_x + ix) * kMemberWords;
-    const int k_use = static_cast<int>(words[MAX_K] & 0xFFu);
-    if (k_use != MAX_K) return;  // a smaller group keeps its members
-    uint32_t member_pos[MAX_K];
+    if ((words[MAX_K] & 0xFFu) != MAX_K) return;  // a smaller group keeps its members
+    const uint32_t member = words[g.sub];
+    const uint32_t max_x = a.width - P, max_y = a.height - P;
+    const float scale = C == 1 ? 3.0f : 1.5f;
+    const float* centre = a.ring + static_cast<size_t>(a.centre_slot) * a.frame_elems;
+    float grid_d = kUnfilled;
+    uint32_t grid_pos = 0;
+    for (int first = 0; first < MAX_K; first += gf) {
+        const uint32_t anchor_packed = __shfl_sync(g.mask, member, first / gf, 8);
+        const uint32_t ax = anchor_packed & 0x1FFFu, ay = (anchor_packed >> 13) & 0x1FFFu;
+        if (g.sub == first) {
+            grid_pos = anchor_packed;
+            grid_d = 0.0f;
+        }
+        held[group][g.sub] = grid_pos;
+        __syncwarp(g.mask);
+        float minus[P * C];
 #pragma unroll
-    for (int m = 0; m < MAX_K; ++m) member_pos[m] = words[m];
-    float grid_d[MAX_K];
-    uint32_t grid_pos[MAX_K];
-    search_volumes<C, GF, COVERS>(g, a, member_pos, C == 1 ? 3.0f : 1.5f, grid_d, grid_pos);
-    bool full = true;
+        for (int r = 0; r < P; ++r)
 #pragma unroll
-    for (int v = 0; v < MAX_K / GF; ++v) full = full && grid_d[v * GF + GF - 1] < kUnfilled;
-    if (!full) return;
-    uint32_t mine = grid_pos[0];
+            for (int c = 0; c < C; ++c)
+                minus[r * C + c] = -__ldg(centre + ((static_cast<size_t>(ay) + r) * a.width + ax + g.sub) * C + c);
+        const uint32_t bx_hi = min(ax / a.blk_step, static_cast<uint32_t>(a.blocks_x - 1));
+        const uint32_t by_hi = min(ay / a.blk_step, static_cast<uint32_t>(a.blocks_y - 1));
+        const uint32_t bx_lo = min(covering_lo(ax, a.blksize, a.blk_step), bx_hi);
+        const uint32_t by_lo = min(covering_lo(ay, a.blksize, a.blk_step), by_hi);
+        for (int t = 0; t < 2 * a.radius; ++t) {
+            const int slot = static_cast<int>(__ldg(a.neighbour_slots + t));
+            const float* frame = a.ring + static_cast<size_t>(slot) * a.frame_elems;
+            const uint32_t packed_t = static_cast<uint32_t>(t + 1) << 26;
+            float frame_d = kUnfilled;
+            uint32_t frame_pos = 0;
+            int searched = 0;
+            for (uint32_t by = by_lo; by <= by_hi && by < by_lo + 4; ++by)
+                for (uint32_t bx = bx_lo; bx <= bx_hi && bx < bx_lo + 4; ++bx) {
+                    const uint32_t block = by * a.blocks_x + bx;
+                    if (!(__ldg(a.confidence + t * a.conf_stride + block) >= a.c_min)) continue;
+                    const int mvx = __ldg(a.mv_field + t * a.mv_stride + block * 2);
+                    const int mvy = __ldg(a.mv_field + t * a.mv_stride + block * 2 + 1);
+                    const uint32_t left = clamp_top_left(static_cast<int>(ax) + mvx - a.refine, max_x);
+                    const uint32_t right = clamp_top_left(static_cast<int>(ax) + mvx + a.refine, max_x);
+                    const uint32_t top = clamp_top_left(static_cast<int>(ay) + mvy - a.refine, max_y);
+                    const uint32_t bottom = clamp_top_left(static_cast<int>(ay) + mvy + a.refine, max_y);
+                    bool contained = false;
+                    for (int i = 0; i < searched; ++i) {
+                        const uint4 r = rects[group][i];
+                        contained |= left >= r.x && right <= r.y && top >= r.z && bottom <= r.w;
+                    }
+                    if (contained) continue;
+                    // The rectangle's best candidate that is not skipped, this lane's share of it first.
+                    float best_d = kUnfilled;
+                    uint32_t best_key = 0xFFFFFFFFu;  // the visiting order: (row, column)
+                    for (uint32_t y0 = top; y0 <= bottom; y0 += kBlk)
+                        for (uint32_t x0 = left; x0 <= right; x0 += kBlk) {
+                            float d[4];
+                            score_block<C>(g, minus, frame, a.width, x0, y0, right, bottom, scale, d);
 #pragma unroll
-    for (int m = 1; m < MAX_K; ++m) mine = g.sub == m ? grid_pos[m] : mine;
-    words[g.sub] = mine;
+                            for (int b = 0; b < 4; ++b) {
+                                const int c = b < 3 ? 8 * b + scattered_candidate(g.sub) : 24;
+                                const uint32_t cx = x0 + c / kBlk, cy = y0 + c % kBlk;
+                                const uint32_t key = cy << 13 | cx;
+                                if (!key_less(d[b], key, best_d, best_key)) continue;
+                                bool skip = false;
+                                for (int i = 0; i < searched; ++i) {
+                                    const uint4 r = rects[group][i];
+                                    skip |= cx >= r.x && cx <= r.y && cy >= r.z && cy <= r.w;
+                                }
+                                for (int k = 0; k < first; ++k) skip |= held[group][k] == (packed_t | key);
+                                if (skip) continue;
+                                best_d = d[b];
+                                best_key = key;
+                            }
+                        }
+                    __syncwarp(g.mask);
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) {
+                        const float other_d = __shfl_xor_sync(g.mask, best_d, o);
+                        const uint32_t other_key = __shfl_xor_sync(g.mask, best_key, o);
+                        if (key_less(other_d, other_key, best_d, best_key)) {
+                            best_d = other_d;
+                            best_key = other_key;
+                        }
+                    }
+                    if (best_d < frame_d) {
+                        frame_d = best_d;
+                        frame_pos = packed_t | best_key;
+                    }
+                    if (g.sub == 0) rects[group][searched] = make_uint4(left, right, top, bottom);
+                    ++searched;
+                    __syncwarp(g.mask);
+                }
+            // Sorted insert into lanes first + 1 .. first + gf - 1, as the reference carries it: what a slot
+            // gives up moves on and passes an equal one that is held.
+            float carry_d = frame_d;
+            uint32_t carry_pos = frame_pos;
+            for (int j = first + 1; j < first + gf; ++j) {
+                const float held_d = __shfl_sync(g.mask, grid_d, j, 8);
+                const uint32_t held_pos = __shfl_sync(g.mask, grid_pos, j, 8);
+                if (!(carry_d < held_d)) continue;
+                if (g.sub == j) {
+                    grid_d = carry_d;
+                    grid_pos = carry_pos;
+                }
+                carry_d = held_d;
+                carry_pos = held_pos;
+            }
+        }
+    }
+    // Every volume's last slot filled: the grid replaces the members.
+    const bool open = (g.sub + 1) % gf == 0 && !(grid_d < kUnfilled);
+    if (__ballot_sync(g.mask, open) & g.mask) return;
+    words[g.sub] = grid_pos;
     if (g.sub == 0) words[MAX_K] = static_cast<uint32_t>(MAX_K) | 0x100u;
 }
 
@@ -740,29 +790,14 @@ cudaError_t launch_centre(const CollabLaunch& a, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <int C, int GF, int COVERS>
-cudaError_t launch_walk(const CollabLaunch& a, cudaStream_t stream) {
-    const int refs_x = (a.width - P + STEP - 1) / STEP + 1, refs_y = (a.height - P + STEP - 1) / STEP + 1;
-    const dim3 grid((refs_x + kGroups - 1) / kGroups, refs_y);
-    collab_walk_kernel<C, GF, COVERS><<<grid, kThreads, 0, stream>>>(a);
-    return cudaGetLastError();
-}
-
-template <int C, int GF>
-cudaError_t launch_walk_covers(const CollabLaunch& a, cudaStream_t stream) {
-    switch ((a.blksize + a.blk_step - 1) / a.blk_step) {
-        case 1: return launch_walk<C, GF, 1>(a, stream);
-        case 2: return launch_walk<C, GF, 2>(a, stream);
-        case 3: return launch_walk<C, GF, 3>(a, stream);
-        default: return launch_walk<C, GF, 4>(a, stream);
-    }
-}
-
 template <int C>
 cudaError_t launch_c(const CollabLaunch& a, cudaStream_t stream) {
     const cudaError_t e = launch_centre<C>(a, stream);
     if (e != cudaSuccess || a.radius == 0 || a.k_max != MAX_K) return e;
-    return a.radius == 1 ? launch_walk_covers<C, 2>(a, stream) : launch_walk_covers<C, 4>(a, stream);
+    const int refs_x = (a.width - P + STEP - 1) / STEP + 1, refs_y = (a.height - P + STEP - 1) / STEP + 1;
+    const dim3 grid((refs_x + kGroups - 1) / kGroups, refs_y);
+    collab_walk_kernel<C><<<grid, kThreads, 0, stream>>>(a, a.radius == 1 ? 2 : 4);
+    return cudaGetLastError();
 }
 
 }  // namespace

@@ -154,3 +154,29 @@ def test_screened_search_picks_the_exact_members(oracle, kind, w, h, c, sr):
     assert np.array_equal(wsum, o_ws)
     assert np.array_equal(accum, o_acc)
     assert np.array_equal(gw.view(np.uint32), o_gw.view(np.uint32))
+
+
+@pytest.mark.parametrize("w,h,c,radius,refine,seed", [(40, 33, 1, 1, 1, 1), (65, 41, 1, 3, 4, 2), (33, 50, 2, 2, 3, 3),
+                                                      (57, 24, 2, 1, 2, 4)])
+def test_walk_keeps_the_reference_order_on_ties(oracle, w, h, c, radius, refine, seed):
+    """Frames of four levels: equal distances within rectangles, between frames and in the volumes' tails,
+    whose order the accumulators' weights depend on; every refine radius, one and two channels."""
+    rng = np.random.default_rng(seed)
+    frames = 2 * radius + 1
+    base = np.round(rng.uniform(0, 3, (h // 4 + 2, w // 4 + 2, c)))
+    ring = np.stack([np.kron(np.roll(base, t, axis=1), np.ones((4, 4, 1)))[:h, :w] for t in range(frames)])
+    ring = (ring + np.round(rng.normal(0, 0.4, ring.shape))).clip(0, 3) / 3
+    bx, by = -(-w // 8), -(-h // 8)
+    case = dict(ring=ring.astype(np.float32).reshape(-1), width=w, height=h, channels=c, centre_slot=radius,
+                radius=radius, c_min=0.2, refine=refine, spatial_radius=6, k_max=8, sigma=(0.05,) * c, lambda_ht=3.0,
+                rho=0.0, kaiser_beta=2.0, mv_field=rng.integers(-5, 6, 2 * radius * bx * by * 2).astype(np.int32),
+                confidence=rng.uniform(0, 1, 2 * radius * bx * by).astype(np.float32),
+                neighbour_slots=np.array([s for s in range(frames) if s != radius], np.uint32),
+                mv_stride=bx * by * 2, conf_stride=bx * by, blocks_x=bx, blocks_y=by)
+    accum, wsum, gw = run_gpu(case)
+    kw = dict(case)
+    o_acc, o_ws, o_gw = oracle.collab_fused(kw.pop("ring"), kw.pop("width"), kw.pop("height"), kw.pop("channels"),
+                                            **kw)
+    assert np.array_equal(wsum, o_ws)
+    assert np.array_equal(accum, o_acc)
+    assert np.array_equal(gw.view(np.uint32), o_gw.view(np.uint32))
