@@ -383,10 +383,14 @@ AvdStatus avd_host_flush(AvdHost* h, AvdHostSink sink, void* user) {
     size_t tail = 0;
     AvdStatus st = avd_engine_finish(h->engine, &tail);
     if (st != AVD_OK) return engine_fail(h, st);
+    // Two frames in flight over the two output sets: the next frame is denoised and read back while the
+    // sink has this one. A frame whose successor fails is still handed over before the failure returns.
+    AvdStatus next = tail > 0 ? emit_into_slot(h, 0) : AVD_OK;
     for (size_t i = 0; i < tail; ++i) {
-        if (AvdStatus e = emit_into_slot(h, 0)) return e;
-        if (AvdStatus e = wait_for(h, 0)) return e;
-        hand_to_sink(h, sink, user, slot_views(h, 0));
+        if (next != AVD_OK) return next;
+        if (i + 1 < tail) next = emit_into_slot(h, (i + 1) % kSets);
+        if (AvdStatus e = wait_for(h, i % kSets)) return e;
+        hand_to_sink(h, sink, user, slot_views(h, i % kSets));
     }
     h->next_out = 0;
     return AVD_OK;
