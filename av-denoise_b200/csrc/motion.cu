@@ -26,7 +26,8 @@
 // block, `mv_stride` values per neighbour; confidence one f32 per block, `conf_stride` per
 // neighbour.
 //
-// Design: one CTA per (block, neighbour); every thread owns one candidate offset and sums its SAD
+// Design, other block sizes (8, 16 and 32 take the row search below): one CTA per (block, neighbour); every
+// thread owns one candidate offset and sums its SAD
 // sequentially in the order above (the sum is bit-identical to the reference's for any grouping of
 // candidates, because each SAD is a sequential f32 sum in a fixed order). The argmin packs
 // (SAD bits, candidate index) into one 64-bit key: non-negative floats order like their bit
@@ -339,22 +340,18 @@ __global__ void __launch_bounds__(((2 * R + 1) * (2 * R + 1) + 31) / 32 * 32) fi
     write_fine(a, bx, by, n, b);
 }
 
-// Register-blocked search for the common block sizes: one warp per (block, neighbour), several
-// blocks per CTA. Each work item is one candidate row and three adjacent offsets along it (five for
-// the wide coarse window of the camera model's first search); per block row it holds BLK + 2 (or
-// BLK + 4) window values in registers and scores the offsets from them, so a SAD term costs well
-// under one shared load instead of two. Every SAD is still the
-// sequential row-major sum, so the vectors are the generic kernels' bit for bit.
+// Register-blocked windows of the escalation, one window to a CTA: each work item is one candidate row and
+// three adjacent offsets along it; per block row it holds BLK + 2 window values in registers and scores the
+// offsets from them, so a SAD term costs well under one shared load instead of two.
 template <int BLK, int R>
 struct Blocked {
     static constexpr int kSide = 2 * R + 1;
-    static constexpr int kWide = R > kMaxRadius ? 5 : 3;  // offsets per work item
+    static constexpr int kWide = 3;  // offsets per work item
     static constexpr int kGroups = (kSide + kWide - 1) / kWide;
     static constexpr int kItems = kSide * kGroups;
     static constexpr int kRows = BLK + 2 * R;
     static constexpr int kReach = kGroups * kWide + BLK - 1;             // columns the last group reads
     static constexpr int kStride = (kReach > kRows ? kReach : kRows) | 1;  // odd: spreads the banks
-    static constexpr int kWarps = BLK >= 32 ? 2 : 4;
     static constexpr int kWindow = kStride * kRows;
 };
 
@@ -393,83 +390,169 @@ __device__ __forceinline__ void blocked_item(int item, const float* centre_tile,
         if (dx0 + k < B::kSide) sads[dy * B::kSide + dx0 + k] = part[k];
 }
 
+// The windowed search for the common block sizes: one lane scores one candidate row of one (block,
+// neighbour) pair, all 2R + 1 offsets of it, and a CTA takes as many pairs as its lanes and shared memory
+// hold (seven at the usual radius 4, 63 of 64 lanes). What bounds it is FP32 issue: two operations per SAD
+// term, which the sequential sums allow no way around. A lane that holds BLK + 2R window samples and a block
+// row in registers spends ten 16-byte shared loads on 144 terms, and its nine sums are independent chains.
+// (Three offsets per item, one warp per pair, spent 18 scalar window loads with two-way bank conflicts on
+// 48 terms, and its lane 0 alone summed the window's mean and bar.)
+// Per launch at 3840x2160, block 16: radius 4 0.52 -> 0.34 ms, radius 2 2.35 -> 1.00 ms,
+// radius 1 0.52 -> 0.24 ms; the coarse level's 8 x 8 blocks 0.196 -> 0.116 ms at radius 4.
+// Every SAD is still the sequential row-major sum, so the vectors are the generic kernels' bit for bit.
 template <int BLK, int R>
-__device__ __forceinline__ void blocked_window(const SearchLevel& L, int64_t centre_base, int64_t nbr_base, int ox,
-                                               int oy, int cdx, int cdy, float* centre_tile, float* window,
-                                               float* sads, int lane, unsigned long long* best_key) {
-    using B = Blocked<BLK, R>;
-    for (int i = lane; i < BLK * BLK; i += 32) {
-        const int py = i / BLK, px = i % BLK;
-        centre_tile[i] = L.pyramid[centre_base + static_cast<int64_t>(clamp_to(oy + py, L.height)) * L.width +
-                                   clamp_to(ox + px, L.width)];
+struct RowSearch {
+    static constexpr int kSide = 2 * R + 1;
+    static constexpr int kSpan = BLK + 2 * R;
+    // Rows of 16-byte chunks, an odd number of them: eight consecutive rows start on different bank groups.
+    // A pair's rows are padded so that the next pair's lanes carry that sequence on.
+    static constexpr int kStride = ((kSpan + 3) / 4 | 1) * 4;
+    static constexpr int kRows = kSpan + ((kSide - kSpan) % 8 + 8) % 8;
+    static constexpr int kCentre = BLK * BLK + 4;
+    static constexpr int kPairBytes = (kCentre + kRows * kStride + kSide * kSide) * 4 + kSide * 8 + 24;
+    static constexpr int kFit = 48 * 1024 / kPairBytes;
+    static constexpr int kPairs = 64 / kSide < kFit ? 64 / kSide : kFit;
+    static constexpr int kThreads = kPairs * kSide <= 32 ? 32 : 64;
+    static_assert(kPairs >= 1 && kPairs <= kThreads, "a pair fits the CTA");
+};
+
+// Rows [0, SPAN) of a SPAN-wide square at (x0, y0), clamped, by the whole CTA: asynchronous copies, so the
+// loads of all a CTA's squares are in flight together (with loads through registers the staging of one
+// square waited for the one before it, and at radii 1 and 2, whose scoring is short, that was the kernel).
+template <int SPAN, int STRIDE, int THREADS>
+__device__ __forceinline__ void stage_square(const float* __restrict__ plane, const SearchLevel& L, int x0, int y0,
+                                             float* out) {
+    constexpr int kLanes = SPAN <= 8 ? 8 : (SPAN <= 16 ? 16 : 32), kStep = THREADS / kLanes;
+    const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(out));
+    for (int x = threadIdx.x % kLanes; x < SPAN; x += kLanes) {
+        const float* col = plane + clamp_to(x0 + x, L.width);
+#pragma unroll 4
+        for (int y = threadIdx.x / kLanes; y < SPAN; y += kStep)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + (y * STRIDE + x) * 4),
+                         "l"(col + static_cast<int64_t>(clamp_to(y0 + y, L.height)) * L.width)
+                         : "memory");
     }
-    const int wx0 = ox + cdx - R, wy0 = oy + cdy - R;
-    for (int i = lane; i < B::kWindow; i += 32) {
-        const int wy = i / B::kStride, wx = i % B::kStride;
-        window[i] = L.pyramid[nbr_base + static_cast<int64_t>(clamp_to(wy0 + wy, L.height)) * L.width +
-                              clamp_to(wx0 + wx, L.width)];
-    }
-    __syncwarp();
-    for (int item = lane; item < B::kItems; item += 32) blocked_item<BLK, R>(item, centre_tile, window, sads);
-    __syncwarp();
-    unsigned long long key = ~0ull;
-    for (int i = lane; i < B::kSide * B::kSide; i += 32) {
-        const float v = sads[i];
-        if (v < kNoSad) {
-            const unsigned long long k = (static_cast<unsigned long long>(__float_as_uint(v)) << 32) | static_cast<unsigned>(i);
-            key = k < key ? k : key;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
-        key = other < key ? other : key;
-    }
-    *best_key = key;
 }
 
 template <int BLK, int R, bool COARSE>
-__global__ void __launch_bounds__(Blocked<BLK, R>::kWarps * 32) blocked_kernel(SearchArgs a) {
-    using B = Blocked<BLK, R>;
-    __shared__ __align__(16) float centre_tiles[B::kWarps][BLK * BLK];
-    __shared__ float windows[B::kWarps][B::kWindow];
-    __shared__ float sad_buf[B::kWarps][B::kSide * B::kSide];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bx = blockIdx.x * B::kWarps + warp, by = blockIdx.y, n = blockIdx.z;
-    if (bx >= a.L.blocks_x) return;  // the whole warp leaves; only warp-scoped syncs follow
-    const int64_t centre_base = a.L.level_base + static_cast<int64_t>(a.centre_slot) * a.L.slot_pixels;
-    const int64_t nbr_base = a.L.level_base + static_cast<int64_t>(search_slot(a, n)) * a.L.slot_pixels;
-    const int ox = bx * a.L.step, oy = by * a.L.step;
-    int cdx = 0, cdy = 0;
-    if (!COARSE && a.use_seed) {
-        const int32_t* mv = a.mv_field + static_cast<int64_t>(n) * a.mv_stride + (by * a.L.blocks_x + bx) * 2;
-        cdx = mv[0];
-        cdy = mv[1];
-    }
+__global__ void __launch_bounds__(RowSearch<BLK, R>::kThreads) row_search_kernel(SearchArgs a) {
+    using B = RowSearch<BLK, R>;
+    constexpr int kSide = B::kSide, kPairs = B::kPairs, kThreads = B::kThreads;
+    __shared__ __align__(16) float centres[kPairs][B::kCentre];
+    __shared__ __align__(16) float windows[kPairs][B::kRows * B::kStride];
+    __shared__ unsigned long long keys[kPairs][kSide];
+    __shared__ float sads[kPairs][kSide * kSide];
+    __shared__ int4 at[kPairs];  // block origin, window centre
+    __shared__ int open[kPairs];
+    const int t = threadIdx.x, n = blockIdx.y;
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * kPairs;
+    const int64_t blocks = static_cast<int64_t>(a.L.blocks_x) * a.L.blocks_y;
+    const int count = blocks - first < kPairs ? static_cast<int>(blocks - first) : kPairs;
+    const float* centre = a.L.pyramid + a.L.level_base + static_cast<int64_t>(a.centre_slot) * a.L.slot_pixels;
+    const float* nbr = a.L.pyramid + a.L.level_base + static_cast<int64_t>(search_slot(a, n)) * a.L.slot_pixels;
     const bool want_mean = !COARSE && a.sad_out != nullptr, want_bar = !COARSE && a.esc_state != nullptr;
-    unsigned long long key;
-    blocked_window<BLK, R>(a.L, centre_base, nbr_base, ox, oy, cdx, cdy, centre_tiles[warp], windows[warp],
-                           sad_buf[warp], lane, &key);
-    WinBest best{cdx, cdy, kNoSad, 0.0f, 0.0f, cdx, cdy};
-    if (lane == 0) best = window_result<R>(sad_buf[warp], key == ~0ull ? -1 : static_cast<int>(key & 0xffffffffu), cdx,
-                                           cdy, want_mean, want_bar);
-    int mdx, mdy;
-    const int scale = COARSE ? a.level_scale : 1;
-    if (model_window(a.predictions, n, ox, oy, BLK, scale, a.L.width, a.L.height, R, cdx, cdy, &mdx, &mdy)) {
-        blocked_window<BLK, R>(a.L, centre_base, nbr_base, ox, oy, mdx, mdy, centre_tiles[warp], windows[warp],
-                               sad_buf[warp], lane, &key);
-        if (lane == 0) {
-            const WinBest ch = window_result<R>(sad_buf[warp], key == ~0ull ? -1 : static_cast<int>(key & 0xffffffffu),
-                                                mdx, mdy, want_mean, want_bar);
-            if (__fadd_rn(ch.sad, model_bias(a, COARSE ? a.floor_scale : 1.0f)) < best.sad) best = ch;
+
+    int bx = 0, by = 0, cdx = 0, cdy = 0;  // of pair t
+    if (t < count) {
+        by = static_cast<int>((first + t) / a.L.blocks_x);
+        bx = static_cast<int>((first + t) % a.L.blocks_x);
+        if (!COARSE && a.use_seed) {
+            const int32_t* mv = a.mv_field + static_cast<int64_t>(n) * a.mv_stride + (by * a.L.blocks_x + bx) * 2;
+            cdx = mv[0];
+            cdy = mv[1];
+        }
+        at[t] = make_int4(bx * a.L.step, by * a.L.step, cdx, cdy);
+    }
+    if (t < kPairs) open[t] = t < count;
+    __syncthreads();
+    for (int p = 0; p < count; ++p)
+        stage_square<BLK, BLK, kThreads>(centre, a.L, at[p].x, at[p].y, centres[p]);
+
+    const int pair = t / kSide, dy = t - pair * kSide;
+    // Every open pair's window staged and scored; its result at thread `pair` index.
+    auto window = [&](int cx, int cy) {
+        for (int p = 0; p < count; ++p) {
+            if (open[p]) stage_square<B::kSpan, B::kStride, kThreads>(nbr, a.L, at[p].x + at[p].z - R,
+                                                                      at[p].y + at[p].w - R, windows[p]);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (pair < count && open[pair]) {
+            float part[kSide];
+#pragma unroll
+            for (int k = 0; k < kSide; ++k) part[k] = 0.0f;
+            constexpr int kChunk = BLK < 16 ? BLK : 16, kReach = (kChunk + 2 * R + 3) / 4 * 4;
+            const float* crow = centres[pair];
+            const float* wrow = windows[pair] + dy * B::kStride;
+#pragma unroll 1
+            for (int iy = 0; iy < BLK; ++iy) {
+#pragma unroll
+                for (int x = 0; x < BLK; x += kChunk) {
+                    float c[kChunk], w[kReach];
+#pragma unroll
+                    for (int q = 0; q < kChunk; q += 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(crow + x + q);
+                        c[q] = v.x, c[q + 1] = v.y, c[q + 2] = v.z, c[q + 3] = v.w;
+                    }
+#pragma unroll
+                    for (int q = 0; q < kReach; q += 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(wrow + x + q);
+                        w[q] = v.x, w[q + 1] = v.y, w[q + 2] = v.z, w[q + 3] = v.w;
+                    }
+#pragma unroll
+                    for (int ix = 0; ix < kChunk; ++ix)
+#pragma unroll
+                        for (int k = 0; k < kSide; ++k)
+                            part[k] = __fadd_rn(part[k], fabsf(__fsub_rn(c[ix], w[ix + k])));
+                }
+                crow += BLK;
+                wrow += B::kStride;
+            }
+            // The row's best: only SADs below the 1e30 start count, and NaN never compares below it.
+            unsigned long long key = ~0ull;
+#pragma unroll
+            for (int k = 0; k < kSide; ++k) {
+                sads[pair][dy * kSide + k] = part[k];
+                if (part[k] < kNoSad) {
+                    const unsigned long long v = (static_cast<unsigned long long>(__float_as_uint(part[k])) << 32) |
+                                                 static_cast<unsigned>(dy * kSide + k);
+                    key = v < key ? v : key;
+                }
+            }
+            keys[pair][dy] = key;
+        }
+        __syncthreads();
+        WinBest r{cx, cy, kNoSad, 0.0f, 0.0f, cx, cy};
+        if (t < count && open[t]) {
+            unsigned long long key = keys[t][0];
+#pragma unroll
+            for (int k = 1; k < kSide; ++k) key = keys[t][k] < key ? keys[t][k] : key;
+            r = window_result<R>(sads[t], key == ~0ull ? -1 : static_cast<int>(key & 0xffffffffu), cx, cy, want_mean,
+                                 want_bar);
+        }
+        return r;
+    };
+
+    WinBest best = window(cdx, cdy);
+    if (a.predictions) {  // uniform across the grid
+        int mdx = 0, mdy = 0;
+        bool again = false;
+        if (t < count)
+            again = model_window(a.predictions, n, bx * a.L.step, by * a.L.step, BLK, COARSE ? a.level_scale : 1,
+                                 a.L.width, a.L.height, R, cdx, cdy, &mdx, &mdy);
+        if (t < count) {
+            open[t] = again;
+            at[t].z = mdx;
+            at[t].w = mdy;
+        }
+        if (__syncthreads_or(again)) {
+            const WinBest ch = window(mdx, mdy);
+            if (again && __fadd_rn(ch.sad, model_bias(a, COARSE ? a.floor_scale : 1.0f)) < best.sad) best = ch;
         }
     }
-    if (lane != 0) return;
-    if (COARSE) {
-        seed_fine_blocks(a, bx, by, n, best.dx, best.dy);
-        return;
-    }
-    write_fine(a, bx, by, n, best);
+    if (t >= count) return;
+    if (COARSE) seed_fine_blocks(a, bx, by, n, best.dx, best.dy);
+    else write_fine(a, bx, by, n, best);
 }
 
 // The fine pass at radius 0 (the HQ confidence pass scores every block where it stands): one thread
@@ -516,14 +599,15 @@ __global__ void __launch_bounds__(128) zero_radius_fine_kernel(SearchArgs a) {
 }
 
 template <int BLK, int R>
-cudaError_t launch_blocked(bool coarse, const SearchArgs& a, dim3 grid, cudaStream_t s) {
-    using B = Blocked<BLK, R>;
-    dim3 g((grid.x + B::kWarps - 1) / B::kWarps, grid.y, grid.z);
+cudaError_t launch_rows(bool coarse, const SearchArgs& a, dim3 grid, cudaStream_t s) {
+    using B = RowSearch<BLK, R>;
+    const int64_t blocks = static_cast<int64_t>(grid.x) * grid.y;
+    dim3 g(static_cast<unsigned>((blocks + B::kPairs - 1) / B::kPairs), grid.z);
     if (coarse) {
-        blocked_kernel<BLK, R, true><<<g, B::kWarps * 32, 0, s>>>(a);
+        row_search_kernel<BLK, R, true><<<g, B::kThreads, 0, s>>>(a);
     } else {
         if constexpr (R <= kMaxRadius) {
-            blocked_kernel<BLK, R, false><<<g, B::kWarps * 32, 0, s>>>(a);
+            row_search_kernel<BLK, R, false><<<g, B::kThreads, 0, s>>>(a);
         } else {
             return cudaErrorInvalidValue;
         }
@@ -533,11 +617,11 @@ cudaError_t launch_blocked(bool coarse, const SearchArgs& a, dim3 grid, cudaStre
 
 template <int R>
 cudaError_t launch_search(bool coarse, const SearchArgs& a, dim3 grid, cudaStream_t s) {
-    if (R >= 1) {
+    if constexpr (R >= 1) {
         switch (a.L.blksize) {
-            case 8: return launch_blocked<8, R>(coarse, a, grid, s);
-            case 16: return launch_blocked<16, R>(coarse, a, grid, s);
-            case 32: return launch_blocked<32, R>(coarse, a, grid, s);
+            case 8: return launch_rows<8, R>(coarse, a, grid, s);
+            case 16: return launch_rows<16, R>(coarse, a, grid, s);
+            case 32: return launch_rows<32, R>(coarse, a, grid, s);
             default: break;
         }
     }

@@ -57,7 +57,23 @@ def gpu_search(lib, ring, w, h, frames, levels, blksize, overlap, radius, channe
     return pyr.cpu().numpy(), mv.cpu().numpy().reshape(n, bx * by, 2), conf.cpu().numpy().reshape(n, bx * by)
 
 
-@pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(map(str, c[:7])))
+# The row search packs 64 // (2 radius + 1) pairs to a CTA (fewer where shared memory ends first): grids of one
+# pair, one under, one over and several CTAs, at the radii and block sizes above that it also serves.
+ROW_CASES = [
+    (9, 7, 3, 1, 16, 8, 4, 1, True),      # 2 x 1 blocks: one CTA, mostly empty
+    (56, 8, 3, 1, 16, 8, 4, 1, True),     # 7 blocks: exactly one CTA
+    (64, 8, 3, 1, 16, 8, 4, 1, True),     # 8 blocks: one past it
+    (168, 9, 3, 2, 16, 8, 1, 1, True),    # 21 x 2 blocks at radius 1
+    (99, 61, 5, 2, 16, 8, 2, 1, True),
+    (61, 45, 3, 2, 8, 4, 1, 1, True),
+    (77, 50, 3, 2, 8, 4, 5, 1, True),
+    (90, 70, 3, 2, 16, 12, 7, 1, True),
+    (130, 70, 3, 2, 32, 16, 4, 1, True),  # shared memory, not lanes, bounds the CTA
+    (100, 64, 3, 2, 16, 8, 8, 1, False),
+]
+
+
+@pytest.mark.parametrize("case", CASES + ROW_CASES, ids=lambda c: "x".join(map(str, c[:7])))
 def test_motion_search_matches_oracle_bit_for_bit(lib, oracle, case):
     w, h, frames, levels, blksize, overlap, radius, channels, confidence = case
     ring = moving_window(w, h, frames, seed=w * 7 + h, channels=channels)
