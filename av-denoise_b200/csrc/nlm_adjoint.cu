@@ -13,7 +13,8 @@
 // passes its gradient to the first offset reaching it; the clamps fold border terms onto the edge
 // pixels, exactly as the forward reads them.
 //
-// Both kernels run on the forward's tile (nlm_tile.cuh): a CTA of 128 threads owns a 32 x TY tile,
+// Patch radii up to kColsMaxPatch run on the column-pair tile (nlm_adjoint_cols.cu). Past it, both kernels
+// run on the offset-pair tile (nlm_tile.cuh): a CTA of 128 threads owns a 32 x TY tile,
 // the frames are staged in shared memory once per pass, and each step takes two offsets (lanes) in
 // packed f32x2 arithmetic with the forward's row-run / column-strip box sums.
 //  - The record kernel is the forward tile with the max weight's first offset tracked: it writes
@@ -33,6 +34,7 @@
 #include <type_traits>
 
 #include "kernels.h"
+#include "nlm_adjoint.cuh"
 #include "nlm_tile.cuh"
 
 namespace avd {
@@ -67,15 +69,6 @@ template <int C, int S, bool FAST>
 __global__ void __launch_bounds__(kThreads) nlm_record_kernel(NlmLaunch a, RecordOut r) {
     nlm_tile<C, S, FAST, true>(a, blockIdx.x, blockIdx.y, &r);
 }
-
-struct GradArgs {
-    NlmLaunch a;  // the window as a ring: centre slot d, pair k's frames k and 2d - k
-    const float* grad_out;
-    const float* records;
-    float* grad_window;
-    float* partials;  // one per tile
-    float h2;
-};
 
 // Per-pixel values of the outputs a thread owns, from the records.
 template <int C, int V>
@@ -411,10 +404,20 @@ __global__ void __launch_bounds__(kThreads) nlm_grad_kernel(GradArgs g) {
     }
 }
 
-__global__ void strength_kernel(const float* partials, int n, float h2, float strength, float* grad_strength) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// The tiles' partials in a fixed order: one CTA, each thread its strided share, then a tree.
+constexpr int kStrengthThreads = 256;
+__global__ void __launch_bounds__(kStrengthThreads) strength_kernel(const float* partials, int n, float h2,
+                                                                    float strength, float* grad_strength) {
+    __shared__ float sums[kStrengthThreads];
     float total = 0.0f;
-    for (int i = 0; i < n; ++i) total += partials[i];
+    for (int i = threadIdx.x; i < n; i += kStrengthThreads) total += partials[i];
+    sums[threadIdx.x] = total;
+    for (int o = kStrengthThreads / 2; o > 0; o >>= 1) {
+        __syncthreads();
+        if (threadIdx.x < o) sums[threadIdx.x] += sums[threadIdx.x + o];
+    }
+    if (threadIdx.x != 0) return;
+    total = sums[0];
     // h2 = K / strength^2, so dh2/dstrength = -2 h2 / strength.
     *grad_strength = total * (-2.0f * h2 / strength);
 }
@@ -464,7 +467,7 @@ cudaError_t launch_adjoint_s(const NlmLaunch& a, const RecordOut& rec, const Gra
     return cudaGetLastError();
 }
 
-template <int C, int S = 0>
+template <int C, int S = kColsMaxPatch + 1>
 cudaError_t dispatch_adjoint(const NlmLaunch& a, const RecordOut& rec, const GradArgs& g, cudaStream_t s) {
     if constexpr (S <= 16) {
         if (a.patch_radius == S) return launch_adjoint_s<C, S>(a, rec, g, s);
@@ -533,9 +536,12 @@ cudaError_t launch_nlm_backward(const NlmBackwardLaunch& l, cudaStream_t s) {
     a.out = nullptr;
     RecordOut rec{l.grad_out, records, l.grad_window + d * frame_elems};
     GradArgs g{a, l.grad_out, records, l.grad_window, partials, l.h2};
-    e = l.channels == 1 ? dispatch_adjoint<1>(a, rec, g, s) : dispatch_adjoint<2>(a, rec, g, s);
+    // The column-pair tile where its runs fit the registers (at 1280x720 luma d = 2 a = 5 s = 2 record and
+    // gradient take 0.48 and 1.40 ms, 0.53 and 2.77 on the offset-pair tile).
+    if (l.patch_radius <= kColsMaxPatch) e = launch_adjoint_cols(a, rec, g, s);
+    else e = l.channels == 1 ? dispatch_adjoint<1>(a, rec, g, s) : dispatch_adjoint<2>(a, rec, g, s);
     if (e != cudaSuccess) return e;
-    strength_kernel<<<1, 32, 0, s>>>(partials, tiles_for(l.width, l.height, l.patch_radius), l.h2, l.strength,
+    strength_kernel<<<1, kStrengthThreads, 0, s>>>(partials, tiles_for(l.width, l.height, l.patch_radius), l.h2, l.strength,
                                      l.grad_strength);
     return cudaGetLastError();
 }

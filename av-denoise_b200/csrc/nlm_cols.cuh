@@ -127,9 +127,11 @@ __device__ __forceinline__ void load_cols(float2* tile, const float* __restrict_
 template <int C, class K>
 struct ColsState {
     Pair<C> ctr[K::RUNW];
-    float2 a[C][K::V];  // sum w * (I - mu) per channel
+    float2 a[C][K::V];  // sum w * (I - level) per channel; with tracking, sum w * (I - the pixel's own)
+    float2 ref[C][K::V];  // with tracking: the pixel's own value
     float2 ws[K::V];    // sum w
     float2 m[K::V];     // min distance (FAST) or max weight (HQ)
+    int2 id[K::V];      // with tracking: the offset reaching m, the first in the forward's order
     float2 conf[K::V];
     const float2* run;           // tile: this thread's run at offset (0, 0)
     const float2* own;           // tile: this thread's first pixel pair at offset (0, 0)
@@ -137,9 +139,21 @@ struct ColsState {
     const float2* hs_in;         // row sums: this thread's strip
 };
 
-// One step: the N offsets (dx .. dx + N - 1, dy), `at` = dy * pitch + dx in pairs.
-template <int C, int S, bool FAST, bool CONF, class K, int N>
-__device__ __forceinline__ void cols_step(ColsState<C, K>& z, int at, float2 kk, float2 scale2, const float (&off)[3]) {
+// Keeps `v` and its offset's id where it beats the best so far, or ties it with an earlier id (frames
+// are walked one after the other, the forward's order interleaves a pair's two).
+template <bool LESS>
+__device__ __forceinline__ void track(float& best, int& best_id, float v, int id) {
+    if ((LESS ? v < best : v > best) || (v == best && id < best_id)) {
+        best = v;
+        best_id = id;
+    }
+}
+
+// One step: the N offsets (dx .. dx + N - 1, dy), `at` = dy * pitch + dx in pairs. TRACK: the ids
+// (id + q id_step) of the best are kept (the adjoint's records).
+template <int C, int S, bool FAST, bool CONF, bool TRACK, class K, int N>
+__device__ __forceinline__ void cols_step(ColsState<C, K>& z, int at, float2 kk, float2 scale2, const float (&off)[3],
+                                          int id, int id_step) {
     constexpr int V = K::V, RUNW = K::RUNW;
     {
         const float2* n = z.run + at * C;
@@ -190,18 +204,29 @@ __device__ __forceinline__ void cols_step(ColsState<C, K>& z, int at, float2 kk,
             if (FAST) {
                 const float2 e = mul2(dist, kk);
                 w = f2(ex2_approx(e.x), ex2_approx(e.y));
-                z.m[k] = f2(fminf(z.m[k].x, dist.x), fminf(z.m[k].y, dist.y));
+                if (TRACK) {
+                    track<true>(z.m[k].x, z.id[k].x, dist.x, id + q * id_step);
+                    track<true>(z.m[k].y, z.id[k].y, dist.y, id + q * id_step);
+                } else {
+                    z.m[k] = f2(fminf(z.m[k].x, dist.x), fminf(z.m[k].y, dist.y));
+                }
             } else {
                 float2 x = fma2(dist, scale2, f2(-off[q], -off[q]));
                 x = f2(fmaxf(x.x, 0.0f), fmaxf(x.y, 0.0f));
                 const float2 e = mul2(x, kk);
                 w = f2(ex2_approx(e.x), ex2_approx(e.y));
                 if (CONF) w = mul2(w, z.conf[k]);
-                z.m[k] = f2(fmaxf(z.m[k].x, w.x), fmaxf(z.m[k].y, w.y));
+                if (TRACK) {
+                    track<false>(z.m[k].x, z.id[k].x, w.x, id + q * id_step);
+                    track<false>(z.m[k].y, z.id[k].y, w.y, id + q * id_step);
+                } else {
+                    z.m[k] = f2(fmaxf(z.m[k].x, w.x), fmaxf(z.m[k].y, w.y));
+                }
             }
             const Pair<C> v = load_pair<C>(p + (k * K::PITCH + q) * C);
 #pragma unroll
-            for (int c = 0; c < C; ++c) z.a[c][k] = fma2(v.c[c], w, z.a[c][k]);
+            for (int c = 0; c < C; ++c)
+                z.a[c][k] = fma2(TRACK ? sub2(v.c[c], z.ref[c][k]) : v.c[c], w, z.a[c][k]);
             z.ws[k] = add2(z.ws[k], w);
         }
     }
@@ -210,9 +235,10 @@ __device__ __forceinline__ void cols_step(ColsState<C, K>& z, int at, float2 kk,
 
 // Rows dy0 .. dy1 - 1 of one frame's window: `skip_centre` leaves out the offset 0 (the single-frame
 // pass, whose noise offsets come from the table `lut`).
-template <int C, int S, bool FAST, bool CONF, class K>
+template <int C, int S, bool FAST, bool CONF, bool TRACK, class K>
 __device__ __forceinline__ void cols_frame(ColsState<C, K>& z, int A, int dy0, int dy1, bool skip_centre,
-                                           const float* __restrict__ lut, float off_pair, float2 kk, float2 scale2) {
+                                           const float* __restrict__ lut, float off_pair, float2 kk, float2 scale2,
+                                           int id_first, int id_step) {
     const int side = 2 * A + 1;
     for (int dy = dy0; dy < dy1; ++dy) {
         int dx = -A;
@@ -226,17 +252,46 @@ __device__ __forceinline__ void cols_frame(ColsState<C, K>& z, int A, int dy0, i
             const int n = left == 4 || (K::Q == 2 && left > 2) ? 2 : min(left, K::Q);
             float off[3] = {off_pair, off_pair, off_pair};
             if (!FAST && skip_centre) {
-                const int o = (dy + A) * side + dx + A;
 #pragma unroll
-                for (int q = 0; q < 3; ++q) off[q] = lut && q < n ? __ldg(lut + o + q) : 0.0f;
+                for (int q = 0; q < 3; ++q)
+                    off[q] = lut && q < n ? __ldg(lut + (dy + A) * side + dx + A + q) : 0.0f;
             }
             const int at = dy * K::PITCH + dx;
-            if (K::Q == 3 && n == 3) cols_step<C, S, FAST, CONF, K, K::Q>(z, at, kk, scale2, off);
-            else if (n == 2) cols_step<C, S, FAST, CONF, K, 2>(z, at, kk, scale2, off);
-            else cols_step<C, S, FAST, CONF, K, 1>(z, at, kk, scale2, off);
+            const int o = (dy + A) * side + dx + A;
+            const int id = TRACK ? id_first + id_step * (skip_centre && o > A * side + A ? o - 1 : o) : 0;
+            if (K::Q == 3 && n == 3) cols_step<C, S, FAST, CONF, TRACK, K, K::Q>(z, at, kk, scale2, off, id, id_step);
+            else if (n == 2) cols_step<C, S, FAST, CONF, TRACK, K, 2>(z, at, kk, scale2, off, id, id_step);
+            else cols_step<C, S, FAST, CONF, TRACK, K, 1>(z, at, kk, scale2, off, id, id_step);
             dx += n;
         }
     }
+}
+
+// The level samples are staged relative to, per channel: just under the tile's darkest pixel. The weighted
+// sum is then of smaller values and keeps bits that one running sum over several hundred offsets would
+// lose, dark pixels' included. The level is a multiple of 1/256 below the samples, so the subtraction is
+// exact and the distances do not change. `two` is shared memory for two pairs; every thread calls it.
+template <int C, class K>
+__device__ __forceinline__ float2 tile_level(const float* __restrict__ centre, int X0, int Y0, int W, int H, float2* two) {
+    const int tid = threadIdx.x, col = tid & (kHalf - 1), y0 = (tid / kHalf) * K::V;
+    float2 mu = f2(1.0f, 1.0f);
+#pragma unroll
+    for (int k = 0; k < K::V; ++k)
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            const float* own = centre + (static_cast<int64_t>(min(Y0 + y0 + k, H - 1)) * W +
+                                         min(X0 + col + l * kHalf, W - 1)) * C;
+            mu = f2(fminf(mu.x, __ldg(own)), C == 2 ? fminf(mu.y, __ldg(own + 1)) : 0.0f);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        mu = f2(fminf(mu.x, __shfl_xor_sync(0xffffffffu, mu.x, o)), fminf(mu.y, __shfl_xor_sync(0xffffffffu, mu.y, o)));
+    if ((tid & 31) == 0) two[tid >> 5] = mu;
+    __syncthreads();
+    mu = f2(fminf(two[0].x, two[1].x), fminf(two[0].y, two[1].y));
+    __syncthreads();
+    return f2(mu.x > 0.0f && mu.x < 1.0f ? floorf(mu.x * 256.0f) * (1.0f / 256.0f) : 0.0f,
+              mu.y > 0.0f && mu.y < 1.0f ? floorf(mu.y * 256.0f) * (1.0f / 256.0f) : 0.0f);
 }
 
 // A share's sums into the kept ones (`first`: they start them), the thread's own sums cleared.
@@ -260,8 +315,10 @@ extern __shared__ __align__(16) float2 cols_smem[];
 // window's rows (frame by frame) are cut into that many shares, whose sums are added in order. CLUSTER:
 // the CTAs of a cluster take one share each (`rank`) and CTA 0 adds and finishes; otherwise this CTA
 // takes them all in turn, with the same sums (a batch's tile equals the frame denoised alone).
-template <int C, int S, bool FAST, class K, bool CLUSTER>
-__device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int tile_y, int rank, int split) {
+// REC: the adjoint's records instead of the output.
+template <int C, int S, bool FAST, class K, bool CLUSTER, bool REC = false>
+__device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int tile_y, int rank, int split,
+                                          const nlm_tile_detail::RecordOut* rec = nullptr) {
     constexpr int V = K::V;
     const int A = a.search_radius, W = a.width, H = a.height;
     const int X0 = tile_x * 2 * kHalf, Y0 = tile_y * K::TY;
@@ -291,35 +348,13 @@ __device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int ti
         z.ws[k] = f2(0.0f, 0.0f);
         z.m[k] = FAST ? f2(__int_as_float(0x7f800000), __int_as_float(0x7f800000)) : f2(0.0f, 0.0f);
         z.conf[k] = f2(1.0f, 1.0f);
+        z.id[k] = make_int2(-1, -1);
 #pragma unroll
         for (int c = 0; c < C; ++c) z.a[c][k] = f2(0.0f, 0.0f);
     }
 
     const float* centre = a.ring + a.slot_centre * a.frame_elems;
-    // Samples are staged less a level just under the tile's darkest pixel: the weighted sum is then of
-    // smaller values and keeps bits that one running sum over several hundred offsets would lose, dark
-    // pixels' included. The level is a multiple of 1/256 below the samples, so the subtraction is exact
-    // and the distances do not change.
-    float2 mu = f2(1.0f, 1.0f);
-    {
-#pragma unroll
-        for (int k = 0; k < V; ++k)
-#pragma unroll
-            for (int l = 0; l < 2; ++l) {
-                const float* own = centre + (static_cast<int64_t>(min(Y0 + y0 + k, H - 1)) * W +
-                                             min(X0 + col + l * kHalf, W - 1)) * C;
-                mu = f2(fminf(mu.x, __ldg(own)), C == 2 ? fminf(mu.y, __ldg(own + 1)) : 0.0f);
-            }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            mu = f2(fminf(mu.x, __shfl_xor_sync(0xffffffffu, mu.x, o)), fminf(mu.y, __shfl_xor_sync(0xffffffffu, mu.y, o)));
-        if (lane == 0) tile[tid >> 5] = mu;
-        __syncthreads();
-        mu = f2(fminf(tile[0].x, tile[1].x), fminf(tile[0].y, tile[1].y));
-        mu = f2(mu.x > 0.0f && mu.x < 1.0f ? floorf(mu.x * 256.0f) * (1.0f / 256.0f) : 0.0f,
-                mu.y > 0.0f && mu.y < 1.0f ? floorf(mu.y * 256.0f) * (1.0f / 256.0f) : 0.0f);
-        __syncthreads();
-    }
+    const float2 mu = tile_level<C, K>(centre, X0, Y0, W, H, tile);
     const int cols = kHalf + 2 * S + 2 * A, side = 2 * A + 1;
     const int all = (2 * a.pairs + 1) * side;  // window rows of the whole tile
     float2* kept = hs + K::HS_PAIRS + tid;  // [(C + 1) V] of this thread, kColsThreads apart
@@ -338,12 +373,24 @@ __device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int ti
         const int pair = (f - 1) >> 1;
         const bool fwd = (f & 1) != 0;
         const int slot = f == 0 ? a.slot_centre : (fwd ? a.slot_fwd[pair] : a.slot_bwd[pair]);
+        // The forward's order: pair by pair and offset by offset, the forward frame at q (an even id),
+        // then the backward frame at -q; the single-frame pass last.
+        const int id_first = 2 * pair * side * side + (fwd ? 0 : 2 * side * side - 1), id_step = fwd ? 2 : -2;
         load_cols<K, C>(tile, a.ring + slot * a.frame_elems, X0 - S - A, Y0 - S - A, K::rows(A), cols, W, H, mu);
         __syncthreads();
         if (f == 0) {
 #pragma unroll
             for (int i = 0; i < K::RUNW; ++i) z.ctr[i] = load_pair<C>(z.run + i * C);
-            cols_frame<C, S, FAST, false, K>(z, A, dy0, dy1, true, a.spatial_lut, off_pair, kk, scale2);
+            if (REC) {
+#pragma unroll
+                for (int k = 0; k < V; ++k) {
+                    const Pair<C> v = load_pair<C>(z.own + k * K::PITCH * C);
+#pragma unroll
+                    for (int c = 0; c < C; ++c) z.ref[c][k] = v.c[c];
+                }
+            }
+            cols_frame<C, S, FAST, false, REC, K>(z, A, dy0, dy1, true, a.spatial_lut, off_pair, kk, scale2,
+                                                  2 * a.pairs * side * side, 1);
         } else if (use_conf) {
             const float* cf = a.conf + (fwd ? a.conf_fwd_off[pair] : a.conf_bwd_off[pair]);
             const int bc0 = min(min(X0 + col, W - 1) / a.conf_step, a.blocks_x - 1);
@@ -353,9 +400,9 @@ __device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int ti
                 const int br = min(min(Y0 + y0 + k, H - 1) / a.conf_step, a.blocks_y - 1);
                 z.conf[k] = f2(__ldg(cf + br * a.blocks_x + bc0), __ldg(cf + br * a.blocks_x + bc1));
             }
-            cols_frame<C, S, FAST, !FAST, K>(z, A, dy0, dy1, false, nullptr, off_pair, kk, scale2);
+            cols_frame<C, S, FAST, !FAST, REC, K>(z, A, dy0, dy1, false, nullptr, off_pair, kk, scale2, id_first, id_step);
         } else {
-            cols_frame<C, S, FAST, false, K>(z, A, dy0, dy1, false, nullptr, off_pair, kk, scale2);
+            cols_frame<C, S, FAST, false, REC, K>(z, A, dy0, dy1, false, nullptr, off_pair, kk, scale2, id_first, id_step);
         }
         __syncthreads();  // every thread is done with this frame's tile
     }
@@ -398,6 +445,41 @@ __device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int ti
         }
         cluster.sync();  // the others' shared memory stays until it is read
         if (rank != 0) return;
+    }
+
+    if constexpr (REC) {
+        // accumulate.rs:175-201 differentiated at each pixel, as the offset-pair tile records it, but for
+        // the output, which is recorded less the tile's level: dL/dh2 sums w (I - out) over every pixel and
+        // offset with much cancellation, and the rounding of `out` was most of its error (the sum of
+        // w (I - own), divided by the denominator, keeps it to the last bits of the difference).
+#pragma unroll
+        for (int l = 0; l < 2; ++l)
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                const int gx = X0 + col + l * kHalf, gy = Y0 + y0 + k;
+                if (gx >= W || gy >= H) continue;
+                const int64_t px = static_cast<int64_t>(gy) * W + gx;
+                const float m = l ? z.m[k].y : z.m[k].x;
+                const float self_weight = a.wref * (FAST ? ex2_approx(m * kk.x) : m);
+                const float den = self_weight + (l ? z.ws[k].y : z.ws[k].x);
+                const float* g = rec->grad_out + px * C;
+                float* gc = rec->grad_centre + px * C;
+                float* r = rec->records + px * nlm_tile_detail::kRecordWords;
+                const bool live = den > 1e-30f;
+                const float inv = live ? 1.0f / den : 0.0f;
+                float gm = 0.0f;
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    const float away = (l ? z.a[c][k].y : z.a[c][k].x) * inv;  // out - own
+                    gc[c] = live ? g[c] * self_weight * inv : g[c];
+                    gm -= g[c] * a.wref * away * inv;
+                    r[c] = (l ? z.ref[c][k].y : z.ref[c][k].x) + away;
+                }
+                r[2] = inv;
+                r[3] = gm;
+                r[4] = __int_as_float(live ? (l ? z.id[k].y : z.id[k].x) : -1);
+            }
+        return;
     }
 
     // Finish (accumulate.rs:175-201), written straight to the output frame.

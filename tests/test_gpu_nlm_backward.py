@@ -39,6 +39,10 @@ def gpu_backward(lib, window, d, a, s, strength, g, wref=1.0, pair_offset=0.0, s
     (64, 48, 2, 1, 3, 1, 6.0, (0.0, 0.0)),         # chroma
     (72, 40, 1, 1, 4, 2, 8.0, (0.003, 0.003)),     # NLMeans-HQ noise offsets
     (40, 33, 1, 0, 7, 3, 12.0, (0.0, 0.0)),        # spatial only, the 640x360 workload's radii
+    (33, 25, 2, 1, 6, 2, 6.0, (0.0, 0.0)),         # one column and row past a tile, two channels, wide pitch
+    (47, 30, 1, 1, 2, 4, 6.0, (0.002, 0.002)),     # the default patch radius, a pair's second half cut
+    (31, 34, 2, 1, 2, 0, 9.0, (0.0, 0.0)),         # no patch: no halo cells
+    (36, 28, 1, 1, 3, 5, 9.0, (0.0, 0.0)),         # past the column-pair tile's radii
 ])
 def test_gpu_adjoint_matches_fp64(lib, oracle, w, h, c, d, a, s, strength, offsets):
     window = frames_for(w + d, w, h, c, 2 * d + 1)
