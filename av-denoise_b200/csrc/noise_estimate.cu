@@ -18,12 +18,17 @@
 //                              state, the derived words and both NLM offset tables.
 //
 // Design. The reference runs the reading as 9 launches over three tagged radix-select batches. Here
-// one CTA of 1024 threads builds the whole reading: it derives every block's values into a small
-// global scratch (L2-resident: at 3840x2160 that is 32,400 blocks), answers each order statistic
-// with an exact 4-pass 8-bit radix select (one warp scans each query's histogram), and writes the
-// reading words into the frame's history slot. The fold is one CTA as well. Order statistics are
+// one cluster of CTAs of 1024 threads builds the whole reading: it derives every block's values into a
+// small global scratch (L2-resident: at 3840x2160 that is 32,400 blocks), answers each order statistic
+// with an exact 4-pass 8-bit radix select (each CTA counts its share, one warp of the cluster adds and
+// scans each query's histograms), and writes the reading words into the frame's history slot. What bounds
+// it is latency, a few dozen dependent passes over all blocks, so the passes are spread over the eight SMs
+// that cluster barriers and distributed shared memory reach (the frame's own chain waits for the
+// reading; with the curve 1.22 -> 0.24 ms at 3840x2160, 0.34 -> 0.12 at 1920x1080, by one CTA and by eight). The fold is one CTA. Order statistics are
 // exact, so the results equal the reference's tagged selects; every other step rounds each multiply
 // and add on its own (this file is built with -fmad=false), as the oracle does.
+
+#include <cooperative_groups.h>
 
 #include <cstdint>
 
@@ -32,9 +37,17 @@
 namespace avd {
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kNB = 16;
 constexpr int kNoiseChannels = 2;
 constexpr int kReadingThreads = 1024;
+// The reading's cluster, from the elements of its longest passes (blocks, or quarters with the curve): past
+// two per thread eight CTAs win, below it the cluster barriers cost more than the passes (by one CTA and by
+// eight: 920 blocks of two channels 50 and 85 us, 2,040 of two 62 and 71, 3,600 of one 71 and 54, 8,160 of
+// one 88 and 43).
+constexpr unsigned kReadingCluster = 8;
+constexpr size_t kReadingSplitFrom = 2 * kReadingThreads;
 constexpr int kReadingWords = 30;
 constexpr uint32_t kExcluded = 0xFFFFFFFFu;
 constexpr float kStaticGate = 1.5f / 255.0f;
@@ -310,17 +323,69 @@ constexpr int kBinQueries = 2 * kCurveBins;
 
 enum SetKind : int { kSetReference, kSetTexture, kSetKept, kSetRho, kSetQuarter };
 
-struct ReadingShared {
-    uint32_t hist[kBinQueries][256];
-    uint32_t prefix[kBinQueries], rank[kBinQueries];
+// Sums over the blocks, then two minima and two maxima (as the complement's minimum).
+struct ReadingCounts {
     uint32_t ref_n[kNoiseChannels], excl_n[kNoiseChannels], tex_n[kNoiseChannels], kept_n[kNoiseChannels],
         acc_n[kNoiseChannels], rho_n;
-    uint32_t ref_min[kNoiseChannels], ref_max[kNoiseChannels];
+    uint32_t quarter_n, bin_n[kCurveBins];
+    uint32_t ref_min[kNoiseChannels], ref_max_not[kNoiseChannels];
+};
+constexpr int kCountWords = sizeof(ReadingCounts) / 4, kMinWords = 2 * kNoiseChannels;
+
+struct ReadingShared : ReadingCounts {  // the whole frame's counts, the same in every CTA
+    __align__(16) uint32_t hist[kBinQueries][256];
+    uint32_t prefix[kBinQueries], rank[kBinQueries];
     float ceiling[kNoiseChannels], threshold[kNoiseChannels];
     uint32_t trusted[kNoiseChannels];
     uint32_t result[kBinQueries];
-    uint32_t quarter_n, bin_n[kCurveBins];
+    ReadingCounts own;  // this CTA's share of them
 };
+
+// The reading's CTAs: a cluster, or (SPLIT false) one alone, which needs no cluster barriers.
+template <bool SPLIT>
+struct ReadingCtas {
+    __device__ static int count() { return SPLIT ? static_cast<int>(cg::this_cluster().num_blocks()) : 1; }
+    __device__ static int rank() { return SPLIT ? static_cast<int>(cg::this_cluster().block_rank()) : 0; }
+    __device__ static void sync() {
+        if (SPLIT) cg::this_cluster().sync();
+        else __syncthreads();
+    }
+    template <typename T>
+    __device__ static T* at(T* own, int r) {  // CTA r's copy of a shared word
+        return SPLIT ? cg::this_cluster().map_shared_rank(own, r) : own;
+    }
+};
+
+// The counts of the whole frame from every CTA's share (complete for the passes before it). Also orders
+// the scratch the CTAs wrote before it.
+template <bool SPLIT>
+__device__ void gather_counts(ReadingShared& sh) {
+    using Ctas = ReadingCtas<SPLIT>;
+    if (SPLIT) __threadfence();
+    else __threadfence_block();
+    Ctas::sync();
+    const int t = threadIdx.x;
+    if (t < kCountWords) {
+        const bool least = t >= kCountWords - kMinWords;
+        uint32_t total = least ? 0xFFFFFFFFu : 0u;
+        for (int r = 0; r < Ctas::count(); ++r) {
+            const uint32_t v = *Ctas::at(reinterpret_cast<uint32_t*>(&sh.own) + t, r);
+            total = least ? min(total, v) : total + v;
+        }
+        reinterpret_cast<uint32_t*>(static_cast<ReadingCounts*>(&sh))[t] = total;
+    }
+    __syncthreads();
+}
+
+// One word's share by the warp: a single atomic for its 32 lanes.
+__device__ __forceinline__ void add_count(uint32_t* word, uint32_t v) {
+    v = __reduce_add_sync(0xFFFFFFFFu, v);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(word, v);
+}
+__device__ __forceinline__ void least(uint32_t* word, uint32_t v) {
+    v = __reduce_min_sync(0xFFFFFFFFu, v);
+    if ((threadIdx.x & 31) == 0) atomicMin(word, v);
+}
 
 __device__ __forceinline__ uint32_t set_key(const BlockScratch& s, int kind, int c, int i) {
     if (kind == kSetQuarter)
@@ -337,19 +402,21 @@ __device__ __forceinline__ uint32_t set_key(const BlockScratch& s, int kind, int
 
 // Exact order statistics by four 8-bit radix passes: query q asks for the element of rank
 // sh.rank[q] among the elements that `element(i, key, first)` assigns to it (element i joins queries
-// first..first+span-1 with `key`, or none when it returns false). One histogram per query, one warp
-// scanning each query's histogram; sh.result[q] receives the key. Lanes of a warp that add to the
+// first..first+span-1 with `key`, or none when it returns false). One histogram per query and CTA, one
+// warp of the cluster adding and scanning each query's; sh.result[q] receives the key. Lanes of a warp that add to the
 // same histogram word add once, by their count: the keys of one set share their top bits, so plain
 // shared atomics would serialise on a few words.
-template <typename Element>
+template <bool SPLIT, typename Element>
 __device__ void radix_select(int n, int nq, int span, ReadingShared& sh, Element element) {
+    using Ctas = ReadingCtas<SPLIT>;
+    const int ctas = Ctas::count(), cta = Ctas::rank();
     const int t = threadIdx.x;
     if (t < nq) sh.prefix[t] = 0;
     uint32_t mask = 0;
     for (int shift = 24; shift >= 0; shift -= 8) {
         for (int i = t; i < nq * 256; i += blockDim.x) (&sh.hist[0][0])[i] = 0;
         __syncthreads();
-        for (int base = 0; base < n; base += blockDim.x) {
+        for (int base = cta * blockDim.x; base < n; base += ctas * blockDim.x) {
             const int i = base + t;
             uint32_t key = 0;
             int first = 0;
@@ -363,40 +430,55 @@ __device__ void radix_select(int n, int nq, int span, ReadingShared& sh, Element
                     atomicAdd(&sh.hist[0][0] + word, static_cast<uint32_t>(__popc(peers)));
             }
         }
-        __syncthreads();
+        Ctas::sync();
+        // Query q is CTA q % ctas's: its warp adds the shares' histograms and tells every CTA.
         const int warp = t / 32, lane = t % 32;
-        for (int q = warp; q < nq; q += blockDim.x / 32) {
-            const uint32_t* h = sh.hist[q];
+        for (int q = warp * ctas + cta; q < nq; q += blockDim.x / 32 * ctas) {
+            uint32_t h[8] = {};
+            for (int r = 0; r < ctas; ++r) {
+                const uint4* share = reinterpret_cast<const uint4*>(Ctas::at(&sh.hist[q][0], r)) + lane * 2;
+                const uint4 a = share[0], b = share[1];
+                h[0] += a.x, h[1] += a.y, h[2] += a.z, h[3] += a.w;
+                h[4] += b.x, h[5] += b.y, h[6] += b.z, h[7] += b.w;
+            }
             uint32_t mine = 0;
-            for (int b = 0; b < 8; ++b) mine += h[lane * 8 + b];
+#pragma unroll
+            for (int b = 0; b < 8; ++b) mine += h[b];
             uint32_t incl = mine;
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
                 if (lane >= o) incl += v;
             }
-            const uint32_t below = incl - mine, rank = sh.rank[q];
+            const uint32_t below = incl - mine, rank = sh.rank[q], prefix = sh.prefix[q];
+            __syncwarp();
             if (rank >= below && rank < incl) {
-                uint32_t seen = below, b = 0;
-                for (; b < 8; ++b) {
-                    if (rank < seen + h[lane * 8 + b]) break;
-                    seen += h[lane * 8 + b];
+                uint32_t seen = below, digit = 0;
+#pragma unroll
+                for (int b = 0; b < 7; ++b) {
+                    if (digit == static_cast<uint32_t>(b) && rank >= seen + h[b]) {
+                        seen += h[b];
+                        digit = b + 1;
+                    }
                 }
-                sh.prefix[q] |= static_cast<uint32_t>(lane * 8 + b) << shift;
-                sh.rank[q] = rank - seen;
+                for (int r = 0; r < ctas; ++r) {
+                    *Ctas::at(&sh.prefix[q], r) = prefix | static_cast<uint32_t>(lane * 8 + digit) << shift;
+                    *Ctas::at(&sh.rank[q], r) = rank - seen;
+                }
             }
         }
         mask |= 0xFFu << shift;
-        __syncthreads();
+        Ctas::sync();
     }
     if (t < nq) sh.result[t] = sh.prefix[t];
     __syncthreads();
 }
 
 // The keys of ranks[0..nq) among one set's elements (all ranks below the set's count).
+template <bool SPLIT>
 __device__ void select_ranks(const BlockScratch& s, int kind, int c, int n, const uint32_t* ranks, int nq,
                              ReadingShared& sh) {
     if (static_cast<int>(threadIdx.x) < nq) sh.rank[threadIdx.x] = ranks[threadIdx.x];
-    radix_select(n, nq, nq, sh, [&](int i, uint32_t& key, int& first) {
+    radix_select<SPLIT>(n, nq, nq, sh, [&](int i, uint32_t& key, int& first) {
         key = set_key(s, kind, c, i);
         first = 0;
         return key != kExcluded;
@@ -411,6 +493,7 @@ __device__ __forceinline__ float quartile_from_pair(float low, float high, uint3
 __device__ __forceinline__ float median_from_pair(float low, float high) { return (low + high) * 0.5f; }
 
 // The median pair and quartile pair of a set of n elements (all four zero for an empty set).
+template <bool SPLIT>
 __device__ void set_pairs(const BlockScratch& s, int kind, int c, int nb, uint32_t n, float out[4],
                           ReadingShared& sh) {
     if (n == 0) {
@@ -418,7 +501,7 @@ __device__ void set_pairs(const BlockScratch& s, int kind, int c, int nb, uint32
         return;
     }
     const uint32_t ranks[4] = {(n - 1) / 2, n / 2, (n - 1) / 4, (n + 2) / 4};
-    select_ranks(s, kind, c, nb, ranks, 4, sh);
+    select_ranks<SPLIT>(s, kind, c, nb, ranks, 4, sh);
     for (int q = 0; q < 4; ++q) out[q] = key_value(sh.result[q]);
     __syncthreads();
 }
@@ -450,23 +533,23 @@ __device__ QuarterRead read_quarter(const float* r, int C, int bw, int bh, int q
     return out;
 }
 
-template <int C>
+template <int C, bool SPLIT>
 __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const float* __restrict__ records, int width,
                                                                        int height, BlockScratch s, uint32_t min_accepted,
                                                                        bool curve, float* __restrict__ reading) {
     __shared__ ReadingShared sh;
     const int t = threadIdx.x;
     const int bxn = (width + kNB - 1) / kNB, byn = (height + kNB - 1) / kNB, nb = bxn * byn;
-    if (t < kNoiseChannels) {
-        sh.ref_n[t] = sh.excl_n[t] = sh.tex_n[t] = sh.kept_n[t] = sh.acc_n[t] = 0;
-        sh.ref_min[t] = 0xFFFFFFFFu;
-        sh.ref_max[t] = 0u;
-    }
-    if (t == 0) sh.rho_n = 0;
+    using Ctas = ReadingCtas<SPLIT>;
+    const int lane_of = Ctas::rank() * blockDim.x + t, lanes = Ctas::count() * blockDim.x;  // of all its CTAs
+    if (t < kCountWords) reinterpret_cast<uint32_t*>(&sh.own)[t] = t >= kCountWords - kMinWords ? 0xFFFFFFFFu : 0u;
     __syncthreads();
 
     // Block derive (sample.rs:143-276).
-    for (int i = t; i < nb; i += blockDim.x) {
+    uint32_t ref_n[C] = {}, excl_n[C] = {}, tex_n[C] = {}, ref_min[C], ref_max_not[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) ref_min[c] = ref_max_not[c] = 0xFFFFFFFFu;
+    for (int i = lane_of; i < nb; i += lanes) {
         const int bx = i % bxn, by = i / bxn;
         const int bw = min(kNB, width - bx * kNB), bh = min(kNB, height - by * kNB);
         const float pixels = static_cast<float>(bw * bh), pairs = static_cast<float>(bh * (bw - 1));
@@ -485,13 +568,13 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
             s.texture[c][i] = r[texture_lane(C, c)];
             flags |= ((candidate ? 1u : 0u) | (measurable ? 2u : 0u)) << (4 * c);
             if (candidate && measurable) {
-                atomicAdd(&sh.ref_n[c], 1u);
                 const uint32_t k = order_key(sigma);
-                atomicMin(&sh.ref_min[c], k);
-                atomicMax(&sh.ref_max[c], k);
-                if (moved) atomicAdd(&sh.tex_n[c], 1u);
+                ref_n[c] += 1;
+                ref_min[c] = min(ref_min[c], k);
+                ref_max_not[c] = min(ref_max_not[c], ~k);
+                if (moved) tex_n[c] += 1;
             } else if (candidate) {
-                atomicAdd(&sh.excl_n[c], 1u);
+                excl_n[c] += 1;
             }
             if (c == 0) {
                 s.mean0[i] = mean;
@@ -502,8 +585,15 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
         s.mean_lag[i] = pairs > 0.0f ? r[2 * C] / pairs : 0.0f;
         s.flags[i] = flags;
     }
-    __threadfence_block();
-    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        add_count(&sh.own.ref_n[c], ref_n[c]);
+        add_count(&sh.own.excl_n[c], excl_n[c]);
+        add_count(&sh.own.tex_n[c], tex_n[c]);
+        least(&sh.own.ref_min[c], ref_min[c]);
+        least(&sh.own.ref_max_not[c], ref_max_not[c]);
+    }
+    gather_counts<SPLIT>(sh);
 
     // The outlier ceilings and moved-texture thresholds (sample.rs:310-360).
     for (int c = 0; c < C; ++c) {
@@ -511,7 +601,7 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
         float ql = 0.0f, qh = 0.0f;
         if (n > 0) {
             const uint32_t ranks[2] = {(n - 1) / 4, (n + 2) / 4};
-            select_ranks(s, kSetReference, c, nb, ranks, 2, sh);
+            select_ranks<SPLIT>(s, kSetReference, c, nb, ranks, 2, sh);
             ql = key_value(sh.result[0]);
             qh = key_value(sh.result[1]);
         }
@@ -519,13 +609,13 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
         const uint32_t tn = sh.tex_n[c];
         if (tn > 0) {
             const uint32_t ranks[1] = {(tn - 1) * 2 / 5};
-            select_ranks(s, kSetTexture, c, nb, ranks, 1, sh);
+            select_ranks<SPLIT>(s, kSetTexture, c, nb, ranks, 1, sh);
             threshold = key_value(sh.result[0]);
         }
         if (t == 0) {
             const float q = quartile_from_pair(ql, qh, n);
             sh.ceiling[c] = n > 0 ? q * kOutlierFactor : 0.0f;
-            const bool spread = n > 0 && key_value(sh.ref_max[c]) > key_value(sh.ref_min[c]);
+            const bool spread = n > 0 && key_value(~sh.ref_max_not[c]) > key_value(sh.ref_min[c]);
             sh.trusted[c] = (sh.excl_n[c] == 0 || spread) ? 1u : 0u;
             sh.threshold[c] = threshold;
         }
@@ -533,7 +623,8 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
     }
 
     // Block accept (sample.rs:362-500).
-    for (int i = t; i < nb; i += blockDim.x) {
+    uint32_t acc_n[C] = {}, kept_n[C] = {}, rho_n = 0;
+    for (int i = lane_of; i < nb; i += lanes) {
         uint32_t flags = s.flags[i];
         const bool moved = flags & 0x100u;
         bool accepted0 = false;
@@ -545,11 +636,11 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
             const bool textured = moved && sh.tex_n[c] > 0 && s.texture[c][i] > sh.threshold[c];
             if (acc) {
                 flags |= 8u << (4 * c);
-                atomicAdd(&sh.acc_n[c], 1u);
+                acc_n[c] += 1;
             }
             if (acc && !textured) {
                 flags |= 4u << (4 * c);
-                atomicAdd(&sh.kept_n[c], 1u);
+                kept_n[c] += 1;
             }
             if (c == 0) accepted0 = acc;
         }
@@ -560,18 +651,23 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
         if (has_rho) {
             flags |= 0x200u;
             s.rho[i] = fminf(fmaxf(rho, 0.0f), 1.0f);
-            atomicAdd(&sh.rho_n, 1u);
+            rho_n += 1;
         }
         s.flags[i] = flags;
     }
-    __threadfence_block();
-    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        add_count(&sh.own.acc_n[c], acc_n[c]);
+        add_count(&sh.own.kept_n[c], kept_n[c]);
+    }
+    add_count(&sh.own.rho_n, rho_n);
+    gather_counts<SPLIT>(sh);
 
     // The sample (sample.rs:562-710).
     float kept[kNoiseChannels][4] = {};
-    for (int c = 0; c < C; ++c) set_pairs(s, kSetKept, c, nb, sh.kept_n[c], kept[c], sh);
+    for (int c = 0; c < C; ++c) set_pairs<SPLIT>(s, kSetKept, c, nb, sh.kept_n[c], kept[c], sh);
     float rho_pair[4];
-    set_pairs(s, kSetRho, 0, nb, sh.rho_n, rho_pair, sh);
+    set_pairs<SPLIT>(s, kSetRho, 0, nb, sh.rho_n, rho_pair, sh);
 
     // The noise curve (kernels/sample.rs:482-510, kernels/curve.rs:37-133, sample.rs:717-803): the
     // quarters of channel-0 accepted blocks that pass the static gates form the quarter set; those
@@ -582,12 +678,8 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
     if (curve) {
         const float sigma_median = median_from_pair(kept[0][0], kept[0][1]);
         const float flat_limit = fmaxf(kFlatFactor * sigma_median * sigma_median, kFlatFloor);
-        if (t < kCurveBins) sh.bin_n[t] = 0;
-        if (t == 0) sh.quarter_n = 0;
-        __syncthreads();
         const int nq = 4 * nb;
-        for (int base = 0; base < nq; base += blockDim.x) {
-            const int i = base + t;
+        for (int i = lane_of; i - t < nq; i += lanes) {  // whole warps: the votes below are theirs
             uint32_t tag = kNoBin;
             if (i < nq) {
                 const int blk = i / 4, bx = blk % bxn, by = blk / bxn;
@@ -599,18 +691,17 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
                 s.quarter_tag[i] = tag;
             }
             const uint32_t members = __ballot_sync(0xFFFFFFFFu, tag & kQuarterMember);
-            if ((t & 31) == 0 && members) atomicAdd(&sh.quarter_n, static_cast<uint32_t>(__popc(members)));
+            if ((t & 31) == 0 && members) atomicAdd(&sh.own.quarter_n, static_cast<uint32_t>(__popc(members)));
             const uint32_t bin = tag & 0xFFu;
             const uint32_t peers = __match_any_sync(0xFFFFFFFFu, bin);
             if (bin < kCurveBins && (t & 31) == __ffs(peers) - 1)
-                atomicAdd(&sh.bin_n[bin], static_cast<uint32_t>(__popc(peers)));
+                atomicAdd(&sh.own.bin_n[bin], static_cast<uint32_t>(__popc(peers)));
         }
-        __threadfence_block();
-        __syncthreads();
+        gather_counts<SPLIT>(sh);
         const uint32_t qn = sh.quarter_n;
         if (qn > 0) {
             const uint32_t ranks[2] = {(qn - 1) / 2, qn / 2};
-            select_ranks(s, kSetQuarter, 0, nq, ranks, 2, sh);
+            select_ranks<SPLIT>(s, kSetQuarter, 0, nq, ranks, 2, sh);
             quarter_median = median_from_pair(key_value(sh.result[0]), key_value(sh.result[1]));
         }
         // Queries 2b and 2b + 1 are bin b's lower and upper median.
@@ -618,7 +709,7 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
             const uint32_t n = sh.bin_n[t / 2];
             sh.rank[t] = n == 0 ? 0 : ((t % 2) ? n / 2 : (n - 1) / 2);
         }
-        radix_select(nq, kBinQueries, 2, sh, [&](int i, uint32_t& key, int& first) {
+        radix_select<SPLIT>(nq, kBinQueries, 2, sh, [&](int i, uint32_t& key, int& first) {
             const uint32_t tag = s.quarter_tag[i];
             const uint32_t bin = tag & 0xFFu;
             if (!(tag & kQuarterMember) || bin >= static_cast<uint32_t>(kCurveBins)) return false;
@@ -631,7 +722,8 @@ __global__ void __launch_bounds__(kReadingThreads) noise_reading_kernel(const fl
                                         : 0.0f;
     }
 
-    if (t == 0) {
+    Ctas::sync();  // no CTA leaves while another reads its share
+    if (lane_of == 0) {
         auto channel_valid = [&](int c) { return c < C && sh.acc_n[c] >= min_accepted && sh.kept_n[c] > 0; };
         const bool valid0 = sh.rho_n > 0 && channel_valid(0);
         const float static_fraction = static_cast<float>(sh.acc_n[0]) / static_cast<float>(nb);
@@ -917,11 +1009,22 @@ cudaError_t launch_noise_reading(const float* records, int channels, int width, 
     b.flags = reinterpret_cast<uint32_t*>(scratch + 9 * nb);
     b.quarter_sigma = scratch + 10 * nb;
     b.quarter_tag = reinterpret_cast<uint32_t*>(scratch + 14 * nb);
-    if (channels == 1)
-        noise_reading_kernel<1><<<1, kReadingThreads, 0, s>>>(records, width, height, b, min_accepted, curve, reading);
-    else
-        noise_reading_kernel<2><<<1, kReadingThreads, 0, s>>>(records, width, height, b, min_accepted, curve, reading);
-    return cudaGetLastError();
+    const bool split = (curve ? 4 * nb : nb) > kReadingSplitFrom;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kReadingCluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(split ? kReadingCluster : 1);
+    cfg.blockDim = dim3(kReadingThreads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = split ? 1 : 0;
+    auto run = [&](auto kernel) {
+        return cudaLaunchKernelEx(&cfg, kernel, records, width, height, b, min_accepted, curve, reading);
+    };
+    if (channels == 1) return split ? run(noise_reading_kernel<1, true>) : run(noise_reading_kernel<1, false>);
+    return split ? run(noise_reading_kernel<2, true>) : run(noise_reading_kernel<2, false>);
 }
 
 cudaError_t launch_noise_fold(const float* records, const float* results, int capacity, int first, int last,

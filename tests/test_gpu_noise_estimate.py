@@ -189,3 +189,22 @@ def test_fold_matches_oracle(lib, oracle, channels, radius, sigma_scale):
         if radius:
             assert np.array_equal(bits(spatial), o_spatial.view(np.uint32))
             assert np.array_equal(bits(pilot), o_pilot.view(np.uint32))
+
+
+# 2,048 elements (blocks, or quarters with the curve) are the most one CTA reads; past them eight share the
+# passes. Blocks: 32 x 16, 27 x 19, 64 x 32, 683 x 3.
+@pytest.mark.parametrize("w,h,channels,curve", [(512, 256, 1, True), (430, 300, 1, True), (1024, 512, 2, False),
+                                                (10920, 45, 2, False), (10920, 45, 2, True)])
+def test_reading_on_both_sides_of_the_split(lib, oracle, w, h, channels, curve):
+    import torch
+
+    cur, prev = noisy_frames(w, h, channels, 2, 5.0, w + h)
+    rec = torch.zeros(lib.avd_noise_records_floats(w, h, channels), device="cuda")
+    now, before = dev(cur), dev(prev)
+    assert lib.avd_noise_temporal_stats(now.data_ptr(), before.data_ptr(), channels, w, h, int(curve), rec.data_ptr(),
+                                        stream()) == 0
+    torch.cuda.synchronize()
+    records = rec.cpu().numpy()
+    got = gpu_reading(lib, records, (0.01, 0.02), channels, w, h, curve).cpu().numpy()
+    want = oracle.noise_reading(records, np.asarray((0.01, 0.02), np.float32), channels, w, h, True, curve)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (got, want)
