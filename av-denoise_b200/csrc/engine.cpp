@@ -208,7 +208,7 @@ class NlmPass final : public Pass {
             if ((e = o.alloc(fe * sizeof(float))) != cudaSuccess) return gpu_failure("output slot", e);
         if ((e = derived_.alloc(16 * sizeof(float))) != cudaSuccess) return gpu_failure("derived words", e);
         // Integer outputs: the list of pixels the exact finish recomputes (nlm_exact.cu) and its count.
-        if (out_.kind != AVD_SAMPLE_F32 && !exact_all_ && (e = fix_.alloc((pixels() + 1) * sizeof(int))) != cudaSuccess)
+        if (out_.kind != AVD_SAMPLE_F32 && !exact_all_ && (e = fix_.alloc((pixels() + 3) * sizeof(int))) != cudaSuccess)
             return gpu_failure("exact-finish list", e);
         // Fixed derived words (nlmeans/denoiser/noise.rs `fixed_derived_values`): the strength and,
         // with an HQ sigma override, the noise offset.
@@ -954,17 +954,24 @@ class NlmPass final : public Pass {
             // Integer outputs: the window kernel flags the pixels within the band of a change of code
             // and the exact finish recomputes them in the reference kernels' order.
             a.fix_count = fix_.as<int>();
-            a.fix_list = fix_.as<int>() + 1;
+            a.fix_list = fix_.as<int>() + 3;
             a.code_max = sample_max_value(out_);
             a.fix_band = kFixBand;
-            if ((e = cudaMemsetAsync(a.fix_count, 0, sizeof(int), stream)) != cudaSuccess)
+            // The exact finish clears them for the next frame; the first frame, and one after a launch that
+            // failed between, clears them itself.
+            if (!fix_clear_ && (e = cudaMemsetAsync(a.fix_count, 0, 2 * sizeof(int), stream)) != cudaSuccess)
                 return gpu_failure("exact-finish count", e);
+            fix_clear_ = false;
         }
         if ((e = launch_nlm(a, stream)) != cudaSuccess) return gpu_failure("nlm launch", e);
-        if (fix_.ptr && (e = launch_nlm_exact(a, stream)) != cudaSuccess) return gpu_failure("exact finish launch", e);
+        if (fix_.ptr) {
+            int* ticket = fix_.as<int>() + 1;
+            if ((e = launch_nlm_exact(a, stream, ticket)) != cudaSuccess) return gpu_failure("exact finish launch", e);
+            fix_clear_ = true;
+        }
         if (timed) {
             timer_.end(stream, start);
-            if (fix_.ptr) timer_.note_count(stream, a.fix_count);
+            if (fix_.ptr) timer_.note_count(stream, fix_.as<int>() + 2);
         }
         *out_slot = slot;
         return std::nullopt;
@@ -1034,6 +1041,7 @@ class NlmPass final : public Pass {
         next_output_slot_ = 0;
         real_pushes_ = 0;
         pushed_ = false;
+        fix_clear_ = false;
         if (measures_) noise_.reset();
     }
 
@@ -1059,7 +1067,8 @@ class NlmPass final : public Pass {
     DeviceBuffer outputs_[2];
     DeviceBuffer derived_;
     DeviceBuffer lut_, pilot_lut_;
-    DeviceBuffer fix_;  // integer outputs: [count, pixel list] of the exact finish
+    DeviceBuffer fix_;  // integer outputs: [count, ticket, last count, pixel list] of the exact finish
+    bool fix_clear_ = false;
     bool exact_all_ = false;
     TuneOptions tune_;
     int window_variant_ = -1;  // the tuned window kernel variant, chosen at the first window launch

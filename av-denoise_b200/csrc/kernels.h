@@ -97,8 +97,10 @@ int nlm_window_variants(int channels, int patch_radius, bool fast);
 // The exact finish (nlm_exact.cu): every pixel of `args.fix_list[0 .. *args.fix_count)` (every pixel
 // of the frame when `fix_list` is null) recomputed in the order and rounding of the FP32 mirror of
 // the reference kernels (row-major patch sums, separately rounded operations, the mirror's own
-// exponential) and written to `args.out`. The kernel reads the count on the device.
-cudaError_t launch_nlm_exact(const NlmLaunch& args, cudaStream_t stream);
+// exponential) and written to `args.out`. The kernel reads the count on the device. With `ticket` (two
+// ints, the first zero) it ends by clearing the count and the ticket for the next frame and leaves the
+// count in the second.
+cudaError_t launch_nlm_exact(const NlmLaunch& args, cudaStream_t stream, int* ticket = nullptr);
 // The FP32 mirror's exponential of `n` floats on the device (its comparison with the oracle).
 cudaError_t launch_exp_mirror(const float* x, float* out, int64_t n, cudaStream_t stream);
 // The band the window kernel flags around each rounding boundary, in normalised units:

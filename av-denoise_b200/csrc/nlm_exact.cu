@@ -41,6 +41,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "exp_mirror.cuh"
 #include "kernels.h"
@@ -51,6 +54,7 @@ namespace {
 
 constexpr int kWarps = 4;               // 128 threads, one pixel per warp
 constexpr int kMaxTplS = 4;             // patch radii with a compile-time tap loop and staged windows
+constexpr int kMaxSmemBytes = 227 * 1024;
 constexpr int kMaxItemFloats = 2048;    // per warp: the weights and products of one batch of passes
 
 __device__ __forceinline__ int clampc(int v, int limit) { return v < 0 ? 0 : (v >= limit ? limit - 1 : v); }
@@ -134,7 +138,7 @@ __host__ __device__ inline int pass_floats(int C, int side, bool pair) {
 // S in 0..kMaxTplS: compile-time patch radius, windows staged per warp; S < 0: any radius, read
 // from the frames.
 template <int C, int S>
-__global__ void __launch_bounds__(kWarps * 32) nlm_exact_kernel(NlmLaunch a, int warp_floats) {
+__global__ void __launch_bounds__(kWarps * 32) nlm_exact_kernel(NlmLaunch a, int warp_floats, int* ticket) {
     extern __shared__ __align__(16) float exact_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int W = a.width, H = a.height;
@@ -429,6 +433,19 @@ __global__ void __launch_bounds__(kWarps * 32) nlm_exact_kernel(NlmLaunch a, int
         }
         cur ^= 1;  // every lane is past this pixel's window reads (the fold's __syncwarp)
     }
+    if (ticket) {
+        // Every CTA has read the count by its own ticket: the last one keeps it beside the ticket and
+        // clears both for the next frame's window, which saves that frame a launch.
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1) {
+                ticket[1] = static_cast<int>(count);
+                *a.fix_count = 0;
+                *ticket = 0;
+            }
+        }
+    }
 }
 
 __global__ void exp_mirror_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t n) {
@@ -436,8 +453,26 @@ __global__ void exp_mirror_kernel(const float* __restrict__ x, float* __restrict
         out[i] = exp_mirror(x[i]);
 }
 
+// Resident CTAs per SM of one kernel, by device and shared memory: the query costs about as much host
+// time as a launch, and an engine asks the same again for every frame.
 template <int C, int S>
-cudaError_t launch_cs(const NlmLaunch& a, int sms, cudaStream_t stream) {
+cudaError_t resident_ctas(int dev, size_t smem, int* per_sm) {
+    static std::mutex lock;
+    static std::map<std::pair<int, size_t>, int> known;
+    std::lock_guard<std::mutex> g(lock);
+    auto it = known.find({dev, smem});
+    if (it == known.end()) {
+        int n = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, nlm_exact_kernel<C, S>, kWarps * 32, smem);
+        if (e != cudaSuccess) return e;
+        it = known.emplace(std::make_pair(dev, smem), n > 0 ? n : 1).first;
+    }
+    *per_sm = it->second;
+    return cudaSuccess;
+}
+
+template <int C, int S>
+cudaError_t launch_cs(const NlmLaunch& a, int dev, int sms, int* ticket, cudaStream_t stream) {
     const int side = 2 * a.search_radius + 1;
     const int R = a.search_radius + a.patch_radius;
     // one batch must hold at least the largest single pass
@@ -445,35 +480,36 @@ cudaError_t launch_cs(const NlmLaunch& a, int sms, cudaStream_t stream) {
                                               (a.pairs) * pass_floats(C, side, true) + pass_floats(C, side, false)));
     const int warp_floats = (S >= 0 ? window_floats(C, R, a.patch_radius) : 0) + max(items, pass_floats(C, side, a.pairs > 0));
     const size_t smem = sizeof(float) * (kWarps * static_cast<size_t>(warp_floats) + 2 * side * side);
+    // The device's own limit, the same for every caller: two engines of different radii share the kernel.
     cudaError_t e = cudaFuncSetAttribute(nlm_exact_kernel<C, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+                                         kMaxSmemBytes);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nlm_exact_kernel<C, S>, kWarps * 32, smem);
+    e = resident_ctas<C, S>(dev, smem, &per_sm);
     if (e != cudaSuccess) return e;
     // Persistent over the pixels: the count is only known on the device.
     const int64_t ctas_all = ((int64_t)a.width * a.height + kWarps - 1) / kWarps;
-    const int64_t slots = static_cast<int64_t>(sms) * (per_sm > 0 ? per_sm : 1);
+    const int64_t slots = static_cast<int64_t>(sms) * per_sm;
     const int grid = static_cast<int>(ctas_all < slots ? ctas_all : slots);
-    nlm_exact_kernel<C, S><<<grid, kWarps * 32, smem, stream>>>(a, warp_floats);
+    nlm_exact_kernel<C, S><<<grid, kWarps * 32, smem, stream>>>(a, warp_floats, a.fix_list ? ticket : nullptr);
     return cudaGetLastError();
 }
 
 template <int C>
-cudaError_t launch_c(const NlmLaunch& a, int sms, cudaStream_t stream) {
+cudaError_t launch_c(const NlmLaunch& a, int dev, int sms, int* ticket, cudaStream_t stream) {
     switch (a.patch_radius) {
-        case 0: return launch_cs<C, 0>(a, sms, stream);
-        case 1: return launch_cs<C, 1>(a, sms, stream);
-        case 2: return launch_cs<C, 2>(a, sms, stream);
-        case 3: return launch_cs<C, 3>(a, sms, stream);
-        case 4: return launch_cs<C, 4>(a, sms, stream);
-        default: return launch_cs<C, -1>(a, sms, stream);
+        case 0: return launch_cs<C, 0>(a, dev, sms, ticket, stream);
+        case 1: return launch_cs<C, 1>(a, dev, sms, ticket, stream);
+        case 2: return launch_cs<C, 2>(a, dev, sms, ticket, stream);
+        case 3: return launch_cs<C, 3>(a, dev, sms, ticket, stream);
+        case 4: return launch_cs<C, 4>(a, dev, sms, ticket, stream);
+        default: return launch_cs<C, -1>(a, dev, sms, ticket, stream);
     }
 }
 
 }  // namespace
 
-cudaError_t launch_nlm_exact(const NlmLaunch& a, cudaStream_t stream) {
+cudaError_t launch_nlm_exact(const NlmLaunch& a, cudaStream_t stream, int* ticket) {
     static_assert(kMaxTplS == 4, "launch_c dispatches radii 0..4 to the staged kernel");
     if (a.search_radius < 0 || a.search_radius > 8 || a.patch_radius < 0 || a.patch_radius > 16 || a.pairs < 0 ||
         a.pairs > kMaxPairs || (a.fix_list != nullptr) != (a.fix_count != nullptr))
@@ -482,8 +518,8 @@ cudaError_t launch_nlm_exact(const NlmLaunch& a, cudaStream_t stream) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    if (a.channels == 1) return launch_c<1>(a, sms, stream);
-    if (a.channels == 2) return launch_c<2>(a, sms, stream);
+    if (a.channels == 1) return launch_c<1>(a, dev, sms, ticket, stream);
+    if (a.channels == 2) return launch_c<2>(a, dev, sms, ticket, stream);
     return cudaErrorInvalidValue;
 }
 
