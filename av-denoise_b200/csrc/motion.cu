@@ -775,27 +775,20 @@ __global__ void __launch_bounds__(64) flag_kernel(EscalateArgs e) {
     e.state[kStateFlag * sec + slot] = (low || on_edge || closest > kNeighbourDisagreement) ? 1.0f : 0.0f;
 }
 
+constexpr int kEscalateThreads = 128;
 // One window of a block of compile-time size BLK by the whole CTA, the result at thread 0: work items of
 // one candidate row and three adjacent offsets, as Blocked has them, over the CTA's threads (radius 8:
 // 102 items on 128 threads, where one thread per candidate takes 320 and two shared loads per term: the
-// escalations of a 12-frame 1279x719 d = 4 stream 14.1 -> 6.2 ms).
+// escalations of a 12-frame 1279x719 d = 4 stream 14.1 -> 5.8 ms; 6.2 with staging loads through registers).
 template <int BLK, int R>
 __device__ __forceinline__ WinBest window_best_blocked(const SearchLevel& L, int64_t centre_base, int64_t nbr_base,
                                                        int ox, int oy, int cdx, int cdy, WindowScratch<R>& w) {
     using B = Blocked<BLK, R>;
     static_assert(B::kWindow <= (kMaxBlk + 2 * R) * (kMaxBlk + 2 * R), "the window scratch holds the blocked rows");
     const int t = threadIdx.x;
-    for (int i = t; i < BLK * BLK; i += blockDim.x) {
-        const int py = i / BLK, px = i % BLK;
-        w.centre_tile[i] = L.pyramid[centre_base + static_cast<int64_t>(clamp_to(oy + py, L.height)) * L.width +
-                                     clamp_to(ox + px, L.width)];
-    }
-    const int wx0 = ox + cdx - R, wy0 = oy + cdy - R;
-    for (int i = t; i < B::kWindow; i += blockDim.x) {
-        const int wy = i / B::kStride, wx = i % B::kStride;
-        w.window[i] = L.pyramid[nbr_base + static_cast<int64_t>(clamp_to(wy0 + wy, L.height)) * L.width +
-                                clamp_to(wx0 + wx, L.width)];
-    }
+    stage_square<BLK, BLK, kEscalateThreads>(L.pyramid + centre_base, L, ox, oy, w.centre_tile);
+    stage_square<B::kRows, B::kStride, kEscalateThreads>(L.pyramid + nbr_base, L, ox + cdx - R, oy + cdy - R, w.window);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     for (int item = t; item < B::kItems; item += blockDim.x)
         blocked_item<BLK, R>(item, w.centre_tile, w.window, w.sads);
@@ -809,7 +802,6 @@ __device__ __forceinline__ WinBest window_best_blocked(const SearchLevel& L, int
 
 // escalate.rs:400-640 (`mc_escalate_search`, `coarse_search`). BLK and CBLK: the block sizes of the two
 // levels where they are the usual 16 and 8 (the blocked windows), or 0 for any size.
-constexpr int kEscalateThreads = 128;
 template <int C, int BLK, int CBLK>
 __global__ void __launch_bounds__(BLK ? kEscalateThreads : ((2 * C + 1) * (2 * C + 1) + 31) / 32 * 32)
     escalate_kernel(EscalateArgs e) {
