@@ -400,7 +400,7 @@ def run_gpu(args) -> None:
                                "chroma spatial a=5 s=2 strength 5 (a luma engine and a chroma engine on two "
                                "streams)", "frames_per_step": FRAMES,
                    "l2": "flushed between steps (256 MiB write)", "parallelism": f"replicas x{world}"},
-        "roofline": {"bound": "sfu", "kernel": "nlm_window_kernel<1,2,fast> (luma, 604 offsets/pixel)",
+        "roofline": {"bound": "sfu", "kernel": "nlm_cols_kernel<1,2,fast> (luma, 604 offsets/pixel)",
                      "achieved": round(achieved, 2), "peak": round(mufu_peak, 2), "unit": "Gex2/s",
                      "frac": round(achieved / mufu_peak, 4),
                      # dram__bytes_read.sum + dram__bytes_write.sum of one launch in an ncu capture of
