@@ -100,8 +100,9 @@ __device__ __forceinline__ bool model_window(const float* predictions, int n, in
 }
 
 // The best offset of one window, at thread 0. `sads` holds every candidate's SAD.
-template <int R>
-__device__ __forceinline__ void window_argmin(const float* sads, unsigned long long* warp_keys, int* best_index) {
+template <int R, int WARPS>
+__device__ __forceinline__ void window_argmin(const float* sads, unsigned long long (&warp_keys)[WARPS],
+                                              int* best_index) {
     constexpr int kSide = 2 * R + 1;
     constexpr int kCand = kSide * kSide;
     const int t = threadIdx.x;
@@ -123,7 +124,7 @@ __device__ __forceinline__ void window_argmin(const float* sads, unsigned long l
     __syncthreads();
     if (t == 0) {
         unsigned long long best = warp_keys[0];
-        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) best = warp_keys[w] < best ? warp_keys[w] : best;
+        for (int w = 1; w < WARPS; ++w) best = warp_keys[w] < best ? warp_keys[w] : best;
         *best_index = best == ~0ull ? -1 : static_cast<int>(best & 0xffffffffu);
     }
 }
@@ -196,19 +197,25 @@ __device__ __forceinline__ WinBest window_result(const float* sads, int best_ind
     return r;
 }
 
+// One thread per candidate, in whole warps: the CTA of the generic windows.
 template <int R>
+constexpr int kCandidateThreads = ((2 * R + 1) * (2 * R + 1) + 31) / 32 * 32;
+
+// THREADS: of the CTA, one key per warp. A CTA may have more warps than its window has candidates.
+template <int R, int THREADS = kCandidateThreads<R>>
 struct WindowScratch {
+    static_assert(THREADS % 32 == 0, "whole warps");
     float centre_tile[kMaxBlk * kMaxBlk];
     float window[(kMaxBlk + 2 * R) * (kMaxBlk + 2 * R)];
     float sads[(2 * R + 1) * (2 * R + 1)];
-    unsigned long long warp_keys[((2 * R + 1) * (2 * R + 1) + 31) / 32];
+    unsigned long long warp_keys[THREADS / 32];
     int best_index;
 };
 
 // One window around (cdx, cdy), the result at thread 0; every thread must call it.
-template <int R>
+template <int R, int THREADS>
 __device__ __forceinline__ WinBest window_best(const SearchLevel& L, int64_t centre_base, int64_t nbr_base, int ox,
-                                               int oy, int cdx, int cdy, WindowScratch<R>& w, bool want_mean,
+                                               int oy, int cdx, int cdy, WindowScratch<R, THREADS>& w, bool want_mean,
                                                bool want_bar) {
     score_window<R>(L, centre_base, nbr_base, ox, oy, cdx, cdy, w.centre_tile, w.window, w.sads);
     window_argmin<R>(w.sads, w.warp_keys, &w.best_index);
@@ -266,10 +273,10 @@ __device__ __forceinline__ WinBest search_candidates(const SearchArgs& a, int bx
     const int64_t cb = a.L.level_base + static_cast<int64_t>(a.centre_slot) * a.L.slot_pixels;
     const int64_t nb = a.L.level_base + static_cast<int64_t>(search_slot(a, n)) * a.L.slot_pixels;
     const int ox = bx * a.L.step, oy = by * a.L.step;
-    WinBest best = window_best<R>(a.L, cb, nb, ox, oy, sdx, sdy, w, want_mean, want_bar);
+    WinBest best = window_best(a.L, cb, nb, ox, oy, sdx, sdy, w, want_mean, want_bar);
     int mdx, mdy;
     if (model_window(a.predictions, n, ox, oy, a.L.blksize, scale, a.L.width, a.L.height, R, sdx, sdy, &mdx, &mdy)) {
-        const WinBest ch = window_best<R>(a.L, cb, nb, ox, oy, mdx, mdy, w, want_mean, want_bar);
+        const WinBest ch = window_best(a.L, cb, nb, ox, oy, mdx, mdy, w, want_mean, want_bar);
         if (threadIdx.x == 0 && __fadd_rn(ch.sad, bias) < best.sad) best = ch;
     }
     return best;
@@ -321,7 +328,7 @@ __device__ __forceinline__ void write_fine(const SearchArgs& a, int bx, int by, 
 }
 
 template <int R>
-__global__ void __launch_bounds__(((2 * R + 1) * (2 * R + 1) + 31) / 32 * 32) coarse_kernel(SearchArgs a) {
+__global__ void __launch_bounds__(kCandidateThreads<R>) coarse_kernel(SearchArgs a) {
     const int bx = blockIdx.x, by = blockIdx.y, n = blockIdx.z;
     const WinBest b = search_candidates<R>(a, bx, by, n, 0, 0, a.level_scale, model_bias(a, a.floor_scale), false, false);
     if (threadIdx.x != 0) return;
@@ -329,7 +336,7 @@ __global__ void __launch_bounds__(((2 * R + 1) * (2 * R + 1) + 31) / 32 * 32) co
 }
 
 template <int R>
-__global__ void __launch_bounds__(((2 * R + 1) * (2 * R + 1) + 31) / 32 * 32) fine_kernel(SearchArgs a) {
+__global__ void __launch_bounds__(kCandidateThreads<R>) fine_kernel(SearchArgs a) {
     const int bx = blockIdx.x, by = blockIdx.y, n = blockIdx.z;
     const int32_t* mv = a.mv_field + static_cast<int64_t>(n) * a.mv_stride + (by * a.L.blocks_x + bx) * 2;
     const int sdx = a.use_seed ? mv[0] : 0;
@@ -629,8 +636,7 @@ cudaError_t launch_search(bool coarse, const SearchArgs& a, dim3 grid, cudaStrea
         zero_radius_fine_kernel<<<dim3((grid.x + 127) / 128, grid.y, grid.z), 128, 0, s>>>(a);
         return cudaGetLastError();
     }
-    constexpr int kCand = (2 * R + 1) * (2 * R + 1);
-    const int threads = ((kCand + 31) / 32) * 32;
+    constexpr int threads = kCandidateThreads<R>;
     if (coarse) {
         coarse_kernel<R><<<grid, threads, 0, s>>>(a);
     } else {
@@ -782,7 +788,8 @@ constexpr int kEscalateThreads = 128;
 // escalations of a 12-frame 1279x719 d = 4 stream 14.1 -> 5.8 ms; 6.2 with staging loads through registers).
 template <int BLK, int R>
 __device__ __forceinline__ WinBest window_best_blocked(const SearchLevel& L, int64_t centre_base, int64_t nbr_base,
-                                                       int ox, int oy, int cdx, int cdy, WindowScratch<R>& w) {
+                                                       int ox, int oy, int cdx, int cdy,
+                                                       WindowScratch<R, kEscalateThreads>& w) {
     using B = Blocked<BLK, R>;
     static_assert(B::kWindow <= (kMaxBlk + 2 * R) * (kMaxBlk + 2 * R), "the window scratch holds the blocked rows");
     const int t = threadIdx.x;
@@ -800,19 +807,21 @@ __device__ __forceinline__ WinBest window_best_blocked(const SearchLevel& L, int
     return r;
 }
 
+template <int C, int BLK>
+constexpr int kEscalateCta = BLK ? kEscalateThreads : kCandidateThreads<C>;
+
 // escalate.rs:400-640 (`mc_escalate_search`, `coarse_search`). BLK and CBLK: the block sizes of the two
 // levels where they are the usual 16 and 8 (the blocked windows), or 0 for any size.
 template <int C, int BLK, int CBLK>
-__global__ void __launch_bounds__(BLK ? kEscalateThreads : ((2 * C + 1) * (2 * C + 1) + 31) / 32 * 32)
-    escalate_kernel(EscalateArgs e) {
-    __shared__ __align__(16) WindowScratch<C> w;
+__global__ void __launch_bounds__(kEscalateCta<C, BLK>) escalate_kernel(EscalateArgs e) {
+    __shared__ __align__(16) WindowScratch<C, kEscalateCta<C, BLK>> w;
     auto coarse_best = [&](int64_t cb, int64_t nb, int ox, int oy, int dx, int dy) {
         if constexpr (CBLK != 0) return window_best_blocked<CBLK, C>(e.Lc, cb, nb, ox, oy, dx, dy, w);
-        else return window_best<C>(e.Lc, cb, nb, ox, oy, dx, dy, w, false, false);
+        else return window_best(e.Lc, cb, nb, ox, oy, dx, dy, w, false, false);
     };
     auto fine_best = [&](int64_t cb, int64_t nb, int ox, int oy, int dx, int dy) {
         if constexpr (BLK != 0) return window_best_blocked<BLK, C>(e.L, cb, nb, ox, oy, dx, dy, w);
-        else return window_best<C>(e.L, cb, nb, ox, oy, dx, dy, w, false, false);
+        else return window_best(e.L, cb, nb, ox, oy, dx, dy, w, false, false);
     };
     __shared__ int coarse_vec[2];
     const int bx = blockIdx.x, by = blockIdx.y, n = blockIdx.z;
@@ -867,14 +876,13 @@ __global__ void __launch_bounds__(BLK ? kEscalateThreads : ((2 * C + 1) * (2 * C
 template <int R>
 cudaError_t launch_escalate(int radius, const EscalateArgs& e, dim3 grid, cudaStream_t s) {
     if (radius == R) {
-        constexpr int kCand = (2 * R + 1) * (2 * R + 1);
         if constexpr (R >= 4) {
             if (e.L.blksize == 16 && (!e.widen || e.Lc.blksize == 8)) {
-                escalate_kernel<R, 16, 8><<<grid, kEscalateThreads, 0, s>>>(e);
+                escalate_kernel<R, 16, 8><<<grid, kEscalateCta<R, 16>, 0, s>>>(e);
                 return cudaGetLastError();
             }
         }
-        escalate_kernel<R, 0, 0><<<grid, ((kCand + 31) / 32) * 32, 0, s>>>(e);
+        escalate_kernel<R, 0, 0><<<grid, kEscalateCta<R, 0>, 0, s>>>(e);
         return cudaGetLastError();
     }
     if constexpr (R < kMaxRadius) {

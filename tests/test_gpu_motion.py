@@ -255,6 +255,9 @@ ESC_CASES = [
     # blksizes outside 8/16/32: the generic fine kernel, then the recorded centres and tracking
     (120, 80, 3, 2, 12, 6, 2, 6, False, 0.02),
     (64, 48, 3, 1, 4, 2, 1, 4, True, 0.02),
+    # the smallest ceiling of the blocked windows: more warps to the CTA than its candidates fill
+    (160, 96, 5, 2, 16, 8, 2, 4, False, 0.02),
+    (75, 50, 3, 1, 16, 8, 3, 4, True, 0.02),
 ]
 
 
