@@ -35,10 +35,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 
 #include "collab_group.cuh"
 #include "kernels.h"
+#include "smem_limit.h"
 
 namespace avd {
 
@@ -778,13 +778,7 @@ template <int C>
 cudaError_t launch_centre(const CollabLaunch& a, cudaStream_t stream) {
     const int refs_x = (a.width - P + STEP - 1) / STEP + 1, refs_y = (a.height - P + STEP - 1) / STEP + 1;
     if (a.spatial_radius < 0 || a.spatial_radius > kMaxRadius) return cudaErrorInvalidValue;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(collab_screen_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(screen_smem<C>(kMaxRadius)));
-    });
-    if (attr_err != cudaSuccess) return attr_err;
+    if (cudaError_t e = allow_smem<collab_screen_kernel<C>>(screen_smem<C>(kMaxRadius))) return e;
     const dim3 grid((refs_x + kRefsX - 1) / kRefsX, (refs_y + kRefsY - 1) / kRefsY);
     collab_screen_kernel<C><<<grid, kScreenThreads, screen_smem<C>(a.spatial_radius), stream>>>(a);
     return cudaGetLastError();

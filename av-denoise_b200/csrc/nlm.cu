@@ -32,10 +32,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 
 #include "kernels.h"
 #include "nlm_tile.cuh"
+#include "smem_limit.h"
 
 namespace avd {
 
@@ -78,13 +78,7 @@ __global__ void __launch_bounds__(kThreads, C == 1 && FAST ? 5 : 4)
 template <int C, int S, bool FAST>
 cudaError_t launch_csf(const NlmLaunch& a, cudaStream_t stream) {
     using K = Cfg<C, S>;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(nlm_window_kernel<C, S, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        200 * 1024);
-    });
-    if (attr_err != cudaSuccess) return attr_err;
+    if (cudaError_t e = allow_smem<nlm_window_kernel<C, S, FAST>>(200 * 1024)) return e;
     dim3 grid((a.width + kTX - 1) / kTX, (a.height + K::TY - 1) / K::TY);
     size_t smem = nlm_smem_bytes<C, S>(a.search_radius, a.pairs, false);
     nlm_window_kernel<C, S, FAST><<<grid, kThreads, smem, stream>>>(a);
@@ -104,13 +98,7 @@ cudaError_t dispatch_s(const NlmLaunch& a, cudaStream_t stream) {
 template <int C, int S, bool FAST>
 cudaError_t batch_csf(const NlmLaunch* jobs, const int* prefix, int njobs, int* counter, int max_a, int max_pairs,
                       cudaStream_t stream) {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(nlm_batch_kernel<C, S, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        200 * 1024);
-    });
-    if (attr_err != cudaSuccess) return attr_err;
+    if (cudaError_t err = allow_smem<nlm_batch_kernel<C, S, FAST>>(200 * 1024)) return err;
     const size_t smem = nlm_smem_bytes<C, S>(max_a, max_pairs, false);
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);

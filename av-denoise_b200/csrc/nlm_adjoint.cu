@@ -30,12 +30,12 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 #include <type_traits>
 
 #include "kernels.h"
 #include "nlm_adjoint.cuh"
 #include "nlm_tile.cuh"
+#include "smem_limit.h"
 
 namespace avd {
 namespace {
@@ -446,21 +446,15 @@ cudaError_t launch_adjoint_s(const NlmLaunch& a, const RecordOut& rec, const Gra
     const dim3 grid((a.width + kTX - 1) / kTX, (a.height + K::TY - 1) / K::TY);
     const size_t rbytes = record_smem_bytes<C, S>(a.search_radius, a.pairs);
     const size_t gbytes = grad_smem_bytes<C, S>(a.search_radius);
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        for (auto f : {nlm_record_kernel<C, S, true>, nlm_record_kernel<C, S, false>})
-            if (attr == cudaSuccess)
-                attr = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        for (auto f : {nlm_grad_kernel<C, S, true>, nlm_grad_kernel<C, S, false>})
-            if (attr == cudaSuccess)
-                attr = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-    });
-    if (attr != cudaSuccess) return attr;
+    constexpr size_t kRecordSmem = 200 * 1024, kGradSmem = 226 * 1024;
     if (a.fast) {
+        if (cudaError_t e = allow_smem<nlm_record_kernel<C, S, true>>(kRecordSmem)) return e;
+        if (cudaError_t e = allow_smem<nlm_grad_kernel<C, S, true>>(kGradSmem)) return e;
         nlm_record_kernel<C, S, true><<<grid, kThreads, rbytes, s>>>(a, rec);
         nlm_grad_kernel<C, S, true><<<grid, kThreads, gbytes, s>>>(g);
     } else {
+        if (cudaError_t e = allow_smem<nlm_record_kernel<C, S, false>>(kRecordSmem)) return e;
+        if (cudaError_t e = allow_smem<nlm_grad_kernel<C, S, false>>(kGradSmem)) return e;
         nlm_record_kernel<C, S, false><<<grid, kThreads, rbytes, s>>>(a, rec);
         nlm_grad_kernel<C, S, false><<<grid, kThreads, gbytes, s>>>(g);
     }

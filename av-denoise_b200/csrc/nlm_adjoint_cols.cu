@@ -29,7 +29,6 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 
 #include "kernels.h"
 #include "nlm_adjoint.cuh"
@@ -341,17 +340,8 @@ template <int C, int S, bool FAST, bool BIG>
 cudaError_t launch_one(const NlmLaunch& a, const RecordOut& rec, const GradArgs& g, cudaStream_t s) {
     using K = ColsOf<C, S, BIG>;
     using T = GradTile<C, S, BIG>;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(nlm_record_cols_kernel<C, S, FAST, BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(K::smem_bytes(kMaxA)));
-        if (attr == cudaSuccess)
-            attr = cudaFuncSetAttribute(nlm_grad_cols_kernel<C, S, FAST, BIG>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(T::grad_bytes(kMaxA)));
-    });
-    if (attr != cudaSuccess) return attr;
+    if (cudaError_t e = allow_smem<nlm_record_cols_kernel<C, S, FAST, BIG>>(K::smem_bytes(kMaxA))) return e;
+    if (cudaError_t e = allow_smem<nlm_grad_cols_kernel<C, S, FAST, BIG>>(T::grad_bytes(kMaxA))) return e;
     const dim3 grid((a.width + 2 * kHalf - 1) / (2 * kHalf), (a.height + K::TY - 1) / K::TY);
     nlm_record_cols_kernel<C, S, FAST, BIG><<<grid, kColsThreads, K::smem_bytes(a.search_radius), s>>>(a, rec);
     nlm_grad_cols_kernel<C, S, FAST, BIG><<<grid, kColsThreads, T::grad_bytes(a.search_radius), s>>>(g);

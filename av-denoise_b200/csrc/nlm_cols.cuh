@@ -29,10 +29,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 
 #include "kernels.h"
 #include "nlm_tile.cuh"
+#include "smem_limit.h"
 
 namespace avd {
 namespace nlm_cols_detail {
@@ -569,13 +569,7 @@ __global__ void __launch_bounds__(kColsThreads, cols_minb<C, S, FAST>())
 template <int C, int S, bool FAST, bool BIG>
 cudaError_t launch_cols_one(const NlmLaunch& a, int split, cudaStream_t stream) {
     using K = ColsOf<C, S, BIG>;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(nlm_cols_kernel<C, S, FAST, BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(K::smem_bytes(kMaxA)));
-    });
-    if (attr_err != cudaSuccess) return attr_err;
+    if (cudaError_t e = allow_smem<nlm_cols_kernel<C, S, FAST, BIG>>(K::smem_bytes(kMaxA))) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((a.width + 2 * kHalf - 1) / (2 * kHalf) * split, (a.height + K::TY - 1) / K::TY);
     cfg.blockDim = dim3(kColsThreads);
@@ -595,14 +589,9 @@ template <int C, int S, bool FAST, bool BIG>
 cudaError_t launch_cols_batch_one(const NlmLaunch* jobs, const int* prefix, int njobs, int* counter, int a,
                                   bool shares, cudaStream_t stream) {
     using K = ColsOf<C, S, BIG>;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(nlm_cols_batch_kernel<C, S, FAST, BIG>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(K::smem_bytes(kMaxA) + sizeof(float2) * K::KEPT_PAIRS));
-    });
-    if (attr_err != cudaSuccess) return attr_err;
+    if (cudaError_t err = allow_smem<nlm_cols_batch_kernel<C, S, FAST, BIG>>(K::smem_bytes(kMaxA) +
+                                                                             sizeof(float2) * K::KEPT_PAIRS))
+        return err;
     const size_t smem = shares ? sizeof(float2) * (K::tile_pairs(a) + K::HS_PAIRS + K::KEPT_PAIRS) : K::smem_bytes(a);
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);

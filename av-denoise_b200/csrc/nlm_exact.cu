@@ -47,6 +47,7 @@
 
 #include "exp_mirror.cuh"
 #include "kernels.h"
+#include "smem_limit.h"
 
 namespace avd {
 
@@ -54,7 +55,7 @@ namespace {
 
 constexpr int kWarps = 4;               // 128 threads, one pixel per warp
 constexpr int kMaxTplS = 4;             // patch radii with a compile-time tap loop and staged windows
-constexpr int kMaxSmemBytes = 227 * 1024;
+constexpr size_t kMaxSmemBytes = 227 * 1024;
 constexpr int kMaxItemFloats = 2048;    // per warp: the weights and products of one batch of passes
 
 __device__ __forceinline__ int clampc(int v, int limit) { return v < 0 ? 0 : (v >= limit ? limit - 1 : v); }
@@ -481,8 +482,7 @@ cudaError_t launch_cs(const NlmLaunch& a, int dev, int sms, int* ticket, cudaStr
     const int warp_floats = (S >= 0 ? window_floats(C, R, a.patch_radius) : 0) + max(items, pass_floats(C, side, a.pairs > 0));
     const size_t smem = sizeof(float) * (kWarps * static_cast<size_t>(warp_floats) + 2 * side * side);
     // The device's own limit, the same for every caller: two engines of different radii share the kernel.
-    cudaError_t e = cudaFuncSetAttribute(nlm_exact_kernel<C, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kMaxSmemBytes);
+    cudaError_t e = allow_smem<nlm_exact_kernel<C, S>>(kMaxSmemBytes);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = resident_ctas<C, S>(dev, smem, &per_sm);

@@ -17,11 +17,11 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 
 #include "exp_mirror.cuh"
 #include "kernels.h"
 #include "nlm_tile.cuh"
+#include "smem_limit.h"
 
 namespace avd {
 
@@ -95,13 +95,7 @@ __global__ void __launch_bounds__(kThreads, C == 1 ? 4 : 3) nlm_ref_window_kerne
 template <int C, int S, bool FAST>
 cudaError_t launch_ref_csf(const NlmLaunch& a, cudaStream_t stream) {
     using K = Cfg<C, S>;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(nlm_ref_window_kernel<C, S, FAST>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    });
-    if (attr_err != cudaSuccess) return attr_err;
+    if (cudaError_t e = allow_smem<nlm_ref_window_kernel<C, S, FAST>>(220 * 1024)) return e;
     dim3 grid((a.width + kTX - 1) / kTX, (a.height + K::TY - 1) / K::TY);
     const size_t smem = nlm_smem_bytes<C, S>(a.search_radius, a.pairs, true);
     if (smem > 220 * 1024) return cudaErrorInvalidValue;
