@@ -948,8 +948,6 @@ class NlmPass final : public Pass {
             *out_slot = slot;
             return std::nullopt;
         }
-        if (window_variant_ < 0) window_variant_ = tune_window(a);
-        a.variant = window_variant_;
         if (fix_.ptr) {
             // Integer outputs: the window kernel flags the pixels within the band of a change of code
             // and the exact finish recomputes them in the reference kernels' order.
@@ -963,6 +961,8 @@ class NlmPass final : public Pass {
                 return gpu_failure("exact-finish count", e);
             fix_clear_ = false;
         }
+        if (window_variant_ < 0) window_variant_ = tune_window(a);
+        a.variant = window_variant_;
         if ((e = launch_nlm(a, stream)) != cudaSuccess) return gpu_failure("nlm launch", e);
         if (fix_.ptr) {
             int* ticket = fix_.as<int>() + 1;
@@ -980,13 +980,12 @@ class NlmPass final : public Pass {
     // tune/driver: the window kernel's variant for this pass's shape, each timed once on this very
     // launch (without the exact-finish list) when the tuner has no choice for the shape yet.
     int tune_window(const NlmLaunch& a) {
-        // "nlm_window2": stores written before the column-pair tile hold choices among other variants.
+        // "nlm_window3": older stores hold choices among other variants.
         char key[160];
-        std::snprintf(key, sizeof(key), "nlm_window2 c%d s%d a%d d%d fast%d conf%d lut%d %dx%d", a.channels,
+        std::snprintf(key, sizeof(key), "nlm_window3 c%d s%d a%d d%d fast%d conf%d lut%d %dx%d", a.channels,
                       a.patch_radius, a.search_radius, a.pairs, a.fast, a.conf ? 1 : 0, a.spatial_lut ? 1 : 0,
                       a.width, a.height);
-        const int variants = a.ref_ring ? 1 : nlm_window_variants(a.channels, a.patch_radius, a.fast != 0);
-        return tuned_variant(tune_, key, variants, [&](int v) {
+        return tuned_variant(tune_, key, nlm_window_variants(a), [&](int v) {
             NlmLaunch t = a;
             t.variant = v;
             t.fix_list = nullptr;

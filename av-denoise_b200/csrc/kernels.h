@@ -73,16 +73,16 @@ struct NlmLaunch {
     int* fix_list;
     int* fix_count;
     float code_max, fix_band;
-    // The window kernel's launch variant, one of nlm_window_variants(). Up to patch radius
-    // kColsMaxPatch: 0 the column-pair tile (nlm_cols.cuh), 1 the same with its tiles shared by twice as
-    // many CTAs, 2 the offset-pair tile (nlm_tile.cuh), the only one past that radius. Variants differ in
-    // the order of the sums over offsets, within the exact finish's band.
+    // The window kernel's launch variant, one of nlm_window_variants(): how many CTAs fewer than fit may
+    // be resident on an SM. The same kernel on the same tiles, so the results keep their bits. A batch's
+    // jobs carry the CTAs a lone launch shares each tile by (cols_split) here.
     int variant;
 };
 
 cudaError_t launch_nlm(const NlmLaunch& args, cudaStream_t stream);
 constexpr int kColsMaxPatch = 4;
-// The column-pair tile, `split` CTAs of a cluster to a tile, without (fast) and with noise offsets.
+// The column-pair tile, `split` CTAs of a cluster to a tile, without (fast) and with noise offsets, in
+// the resident CTAs of args.variant.
 cudaError_t launch_nlm_cols_fast(const NlmLaunch& args, int split, cudaStream_t stream);
 cudaError_t launch_nlm_cols_hq(const NlmLaunch& args, int split, cudaStream_t stream);
 cudaError_t launch_nlm_cols_batch_fast(const NlmLaunch* jobs, const int* prefix, int njobs, int* counter, int channels,
@@ -92,7 +92,10 @@ cudaError_t launch_nlm_cols_batch_hq(const NlmLaunch* jobs, const int* prefix, i
 // The CTAs a lone launch shares each tile by; a batch's jobs carry it in `variant` (`shares`: some job's
 // is above 1).
 int cols_split(const NlmLaunch& args);
-int nlm_window_variants(int channels, int patch_radius, bool fast);
+// Whether the launch runs the column-pair tile (nlm_cols.cuh), the offset-pair tile (nlm_tile.cuh)
+// otherwise. A matter of sizes alone, and of `fix_count`: see nlm.cu.
+bool runs_cols(const NlmLaunch& args);
+int nlm_window_variants(const NlmLaunch& args);
 
 // The exact finish (nlm_exact.cu): every pixel of `args.fix_list[0 .. *args.fix_count)` (every pixel
 // of the frame when `fix_list` is null) recomputed in the order and rounding of the FP32 mirror of

@@ -134,21 +134,45 @@ int nlm_tile_rows(int /*channels*/, int patch_radius) {
 
 int nlm_tile_cols() { return kTX; }
 
-int nlm_window_variants(int /*channels*/, int patch_radius, bool /*fast*/) {
-    return patch_radius <= kColsMaxPatch ? 3 : 1;
+namespace {
+int frame_tiles(const NlmLaunch& a) {
+    const int rows = nlm_tile_rows(a.channels, a.patch_radius);
+    return ((a.width + kTX - 1) / kTX) * ((a.height + rows - 1) / rows);
+}
+// The rules on tiles below are part of what a launch computes (the order of its sums), so they take the
+// SMs of the one GPU this library is built for, not those of the device it finds.
+constexpr int kSms = 148;
+}  // namespace
+
+// The tile depends on the sizes alone, never on a timing: the two tiles add up the offsets in different
+// orders. Past kColsMaxPatch only the offset-pair tile is built. It also takes a single frame's small
+// window on a small frame, where the column-pair tile's CTAs of 64 threads have too little work to share
+// (a = 2, s = 4, luma: 13 us against 16 at 320x180, 17 and 17 at 640x360, 25 and 21 at 957x539; a = 3,
+// s = 1, chroma: 20 and 22 at 256x144, 24 and 30 at 640x360, 46 and 44 at 957x539), but for integer
+// outputs only: the exact finish gives those the reference's order, while float outputs have to equal a
+// batch's, which runs the column-pair tile.
+bool runs_cols(const NlmLaunch& a) {
+    if (a.patch_radius > kColsMaxPatch || (a.channels != 1 && a.channels != 2)) return false;
+    return !(a.fix_count && a.pairs == 0 && a.search_radius <= 3 && frame_tiles(a) <= 2 * kSms);
 }
 
+int nlm_window_variants(const NlmLaunch& a) { return !a.ref_ring && runs_cols(a) ? 3 : 1; }
+
 // How many CTAs of a cluster share a column-pair tile. A frame's tiles alone leave SMs idle below a few
-// CTAs each: from 3 to an SM on, one CTA per tile (957x539 chroma, 690 tiles: 121 us alone, 129 shared
-// by two); under that, the fewest that reach it, up to the 8 of a portable cluster (640x360, 300 tiles,
-// a = 7: 88 us alone, 69 by two, 80 by four; 203x117, 35 tiles, d = 1 a = 5: 118 alone, 70, 45, 35 by
-// eight), as long as each keeps about two window rows of work for the frames it stages.
+// CTAs each: from 3 to an SM on, one CTA per tile (957x539 chroma a = 5, 690 tiles: 121 us alone, 129
+// shared by two); under that, the fewest that reach it, up to the 8 of a portable cluster (640x360, 300
+// tiles, a = 7: 88 us alone, 69 by two, 80 by four; 203x117, 35 tiles, d = 1 a = 5: 118 alone, 70, 45, 35
+// by eight), as long as the window's rows leave each two after the four that a share's staging is worth
+// (a = 2, one frame: 5 rows, 15 us alone and 17 by two at 256x144; a = 3, 7 rows: 24, 21 by two, 20 by
+// four). Long windows are shared up to 10 tiles to an SM, where the last wave of whole tiles costs more
+// than staging a frame twice (d = 4 a = 4 s = 4: 1100x620 595 us alone, 503 by two; 1279x719 678 and 613;
+// 1920x1080, 2,700 tiles, 1,345 and 1,296).
 int cols_split(const NlmLaunch& a) {
-    const int tiles = ((a.width + kTX - 1) / kTX) * ((a.height + nlm_tile_rows(a.channels, a.patch_radius) - 1) /
-                                                     nlm_tile_rows(a.channels, a.patch_radius));
-    const int rows = (2 * a.pairs + 1) * (2 * a.search_radius + 1);
+    const int tiles = frame_tiles(a), rows = (2 * a.pairs + 1) * (2 * a.search_radius + 1);
     int split = 1;
-    while (split < 8 && tiles * split < 3 * 148 && rows >= 4 * split) split *= 2;
+    while (split < 8 && ((tiles * split < 3 * kSms && rows >= 2 * split + 4) ||
+                         (tiles * split < 10 * kSms && rows >= 40 * split)))
+        split *= 2;
     return split;
 }
 
@@ -172,13 +196,9 @@ cudaError_t launch_nlm(const NlmLaunch& a, cudaStream_t stream) {
         a.patch_radius > 16)
         return cudaErrorInvalidValue;
     if (a.ref_ring) return launch_nlm_ref(a, stream);
-    if (a.patch_radius <= kColsMaxPatch && (a.channels == 1 || a.channels == 2) && a.variant != 2) {
+    if (runs_cols(a)) {
         const int split = cols_split(a);
-        // Variant 1: tiles shared by twice as many CTAs, which evens out the last wave of a long window
-        // (1279x719 d = 4 a = 4: 665 us with one CTA per tile, 605 with two).
-        const int rows = (2 * a.pairs + 1) * (2 * a.search_radius + 1);
-        const int use = a.variant == 1 && split < 8 && rows >= 2 * split ? 2 * split : split;
-        return a.fast ? launch_nlm_cols_fast(a, use, stream) : launch_nlm_cols_hq(a, use, stream);
+        return a.fast ? launch_nlm_cols_fast(a, split, stream) : launch_nlm_cols_hq(a, split, stream);
     }
     if (a.channels == 1) return dispatch_s<1, 0>(a, stream);
     if (a.channels == 2) return dispatch_s<2, 0>(a, stream);

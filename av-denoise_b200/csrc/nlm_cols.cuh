@@ -53,7 +53,7 @@ constexpr int kColsMaxS = kColsMaxPatch;
 constexpr int kColsThreads = 64;
 constexpr int kHalf = 16;      // columns between a pair's lanes
 constexpr int kSmallA = 5, kMaxA = 8;
-constexpr int kMaxSplit = 8;   // CTAs that share a tile (a portable cluster)
+constexpr int kResidencies = 3;  // the tuner's choices of resident CTAs per SM: as many as fit, one or two fewer
 constexpr int kHsPitch = 18;   // row sums: 9 x 16 bytes, an odd number, so 8 rows' stores miss each other
 
 // Q offsets per step; BIG: search radii past 5.
@@ -569,11 +569,21 @@ __global__ void __launch_bounds__(kColsThreads, cols_minb<C, S, FAST>())
 template <int C, int S, bool FAST, bool BIG>
 cudaError_t launch_cols_one(const NlmLaunch& a, int split, cudaStream_t stream) {
     using K = ColsOf<C, S, BIG>;
-    if (cudaError_t e = allow_smem<nlm_cols_kernel<C, S, FAST, BIG>>(K::smem_bytes(kMaxA))) return e;
+    // Shared memory that leaves room for `n` CTAs on an SM (228 KB, 1 KB of it the runtime's per CTA).
+    constexpr auto room = [](int n) { return static_cast<size_t>(228 / n - 1) * 1024; };
+    constexpr int kMinb = cols_minb<C, S, FAST>();
+    constexpr size_t kFewest = room(kMinb - (kResidencies - 1));
+    constexpr size_t kMost = kFewest > K::smem_bytes(kMaxA) ? kFewest : K::smem_bytes(kMaxA);
+    if (cudaError_t e = allow_smem<nlm_cols_kernel<C, S, FAST, BIG>>(kMost)) return e;
+    size_t smem = K::smem_bytes(a.search_radius);
+    if (a.variant > 0 && a.variant < kResidencies) {
+        const size_t least = room(kMinb - a.variant);
+        smem = smem > least ? smem : least;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((a.width + 2 * kHalf - 1) / (2 * kHalf) * split, (a.height + K::TY - 1) / K::TY);
     cfg.blockDim = dim3(kColsThreads);
-    cfg.dynamicSmemBytes = K::smem_bytes(a.search_radius);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute cluster[1];
     cluster[0].id = cudaLaunchAttributeClusterDimension;
