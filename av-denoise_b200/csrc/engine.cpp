@@ -208,8 +208,14 @@ class NlmPass final : public Pass {
             if ((e = o.alloc(fe * sizeof(float))) != cudaSuccess) return gpu_failure("output slot", e);
         if ((e = derived_.alloc(16 * sizeof(float))) != cudaSuccess) return gpu_failure("derived words", e);
         // Integer outputs: the list of pixels the exact finish recomputes (nlm_exact.cu) and its count.
-        if (out_.kind != AVD_SAMPLE_F32 && !exact_all_ && (e = fix_.alloc((pixels() + 3) * sizeof(int))) != cudaSuccess)
-            return gpu_failure("exact-finish list", e);
+        if (out_.kind != AVD_SAMPLE_F32 && !exact_all_) {
+            // The count is zero between frames from here on, whatever becomes of the launches in between
+            // (a push captured into a graph that never runs, for one): an index past the list never forms.
+            e = fix_.alloc((pixels() + 3) * sizeof(int));
+            if (e == cudaSuccess) e = cudaMemset(fix_.ptr, 0, 3 * sizeof(int));
+            if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+            if (e != cudaSuccess) return gpu_failure("exact-finish list", e);
+        }
         // Fixed derived words (nlmeans/denoiser/noise.rs `fixed_derived_values`): the strength and,
         // with an HQ sigma override, the noise offset.
         float words[16] = {0};
@@ -955,8 +961,8 @@ class NlmPass final : public Pass {
             a.fix_list = fix_.as<int>() + 3;
             a.code_max = sample_max_value(out_);
             a.fix_band = kFixBand;
-            // The exact finish clears them for the next frame; the first frame, and one after a launch that
-            // failed between, clears them itself.
+            // The exact finish clears them for the next frame; a frame after a launch that failed between
+            // clears them itself.
             if (!fix_clear_ && (e = cudaMemsetAsync(a.fix_count, 0, 2 * sizeof(int), stream)) != cudaSuccess)
                 return gpu_failure("exact-finish count", e);
             fix_clear_ = false;
@@ -1040,7 +1046,6 @@ class NlmPass final : public Pass {
         next_output_slot_ = 0;
         real_pushes_ = 0;
         pushed_ = false;
-        fix_clear_ = false;
         if (measures_) noise_.reset();
     }
 
@@ -1067,7 +1072,7 @@ class NlmPass final : public Pass {
     DeviceBuffer derived_;
     DeviceBuffer lut_, pilot_lut_;
     DeviceBuffer fix_;  // integer outputs: [count, ticket, last count, pixel list] of the exact finish
-    bool fix_clear_ = false;
+    bool fix_clear_ = true;
     bool exact_all_ = false;
     TuneOptions tune_;
     int window_variant_ = -1;  // the tuned window kernel variant, chosen at the first window launch

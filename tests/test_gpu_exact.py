@@ -114,3 +114,29 @@ def test_exact_hq_chroma_floats(oracle):
 def test_exact_prefilters_floats(oracle, kind):
     pf = avd.PrefilterMode.bilateral(1.5, 0.1) if kind == "bilateral" else avd.PrefilterMode.nlm_spatial(1.5)
     run_exact(oracle, 64, 40, fast(1, 3, 2, 12.0, prefilter=pf), False, 1, 3, 2, 12.0, seed=9, prefilter=pf)
+
+
+def test_a_push_that_never_runs_leaves_the_list_empty():
+    """The first push of an integer engine captured into a graph that is dropped: the count of the exact
+    finish's list is still zero, and the frames pushed after it are the ones a fresh engine gives."""
+    import torch
+
+    w, h = 72, 40
+    u8 = avd.SampleFormat.u8()
+    spec = avd.EngineSpec.nlmeans(fast(0, 2, 2, 6.0), None, avd.Geometry(w, h, avd.ChromaLayout.GRAY, u8, u8))
+    off = avd.TuningConfig(mode="off")
+    frames = clip(w, h, 3, seed=21)
+    want = Runner(spec, off).run(frames)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        late = Runner(spec, off)
+        bufs, planes = late.planes_for(frames[0], u8)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            assert late.engine.push(planes) == 1
+            late.engine.emit_into(late.out_planes())
+        del graph
+        got = late.run(frames[1:])
+    for a, b in zip(got, want[1:]):
+        assert np.array_equal(a[0], b[0])
