@@ -11,7 +11,7 @@
 // the tensor cores: with samples c, n in units of codes around the middle code, exact in f16,
 //     sum c^2 - D = 2 sum c n - sum n^2
 // is a contraction over the 64 (128) samples of a patch whose f32 accumulation is the integer itself
-// or within a known bound of it. The larger of it ranks the smaller distance. Every thread keeps the
+// or within a measured bound of it. The larger of it ranks the smaller distance. Every thread keeps the
 // largest score of its own share of a patch's candidates (64 shares to a patch); the eighth largest of
 // those shares' maxima is reached by at least eight candidates, so a candidate whose score lies below
 // it by more than the error of both scores cannot be among the best eight. A second round of the same
@@ -20,10 +20,11 @@
 // (flat areas full of ties) and every patch of a tile whose samples overrun f16 goes through the exact
 // search of the whole window.
 //
-// The error of a score, in units of squared codes: the tensor core's accumulation (k16 steps of sums
-// below 3 * 64 C R^2, R the largest sample of the tile), the f32 distance's own rounding (1e-5 of it,
-// and the quotients' 2^-24 per sample), and, where the ring holds floats rather than codes, the samples'
-// rounding to f16: |sqrt(D) - sqrt(D~)| is at most the norm of the rounding of both patches.
+// The error of a score, in units of squared codes: the tensor core's accumulation and the sums of squares
+// (screen_score.cuh, which also says what that rests on), the f32 distance's own rounding (1e-5 of it),
+// where the ring holds codes the rounding of their quotients (2^-24 of the largest code per sample), and
+// where it holds floats the samples' rounding to f16: |sqrt(D) - sqrt(D~)| is at most the norm of the
+// rounding of both patches.
 //
 // How. A CTA owns 8 x 4 reference patches (step 4), four groups of 8 (4 x 2) that share a staged tile of
 // 16-byte chunks, chunk (x, y) holding the eight samples x..x+7 of row y: patch row r of candidate
@@ -38,6 +39,7 @@
 
 #include "collab_group.cuh"
 #include "kernels.h"
+#include "screen_score.cuh"
 #include "smem_limit.h"
 
 namespace avd {
@@ -45,6 +47,7 @@ namespace avd {
 namespace {
 
 using namespace collab_detail;
+using screen::mma_f16;
 
 // The lane's share of the distance from `ref` (its 8 x C column) to the candidate at (x, y).
 template <int C>
@@ -233,13 +236,6 @@ __host__ __device__ inline size_t screen_smem(int r) {
     return 16 * C * rows * cp + sizeof(float) * (sums > shares ? sums : shares) +
            sizeof(float) * screen_rows(r) * cp + sizeof(float) * kRefs + sizeof(int) * kRefs +
            sizeof(uint16_t) * kRefs * kList;
-}
-
-__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0,
-                                        float c1, float c2, float c3) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
@@ -490,9 +486,10 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
                 const float n = 64.0f * C;
                 const float reach = 3.0f * n * worst * worst;  // no partial sum is larger
                 const float dist = fmaxf(-sums[qy * cp + qx] - eighth, 0.0f);
-                const float fixed = 4.0f + reach * (static_cast<float>(4 * C + 1) * 2.4e-7f);
+                const float fixed = 4.0f + screen::score_error<C>(reach);
                 const float dist1 = dist + fixed;
-                const float quotients = 4e-4f * sqrtf(n * dist1) + 1e-5f * dist1;
+                // |D - D~| <= 2 sqrt(D) times the norm of the quotients' rounding, 2 * 2^-24 to_code a sample.
+                const float quotients = (codes ? 4.0f * screen::kUlp * to_code * sqrtf(n * dist1) : 0.0f) + 1e-5f * dist1;
                 const float halves = codes ? 0.0f : 2.0f * sqrtf(n) * worst * 4.9e-4f;
                 const float slack = 2.0f * (fixed + quotients) + 4.0f * halves * (sqrtf(dist1) + halves);
                 line[ref] = fmaxf(eighth - slack, -1e29f);
