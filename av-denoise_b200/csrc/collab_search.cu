@@ -16,9 +16,20 @@
 // those shares' maxima is reached by at least eight candidates, so a candidate whose score lies below
 // it by more than the error of both scores cannot be among the best eight. A second round of the same
 // products lists the candidates at or above that line, and the 8-lane group of the patch scores the
-// listed ones (nine or ten of 1,089 on noisy frames) in the exact order. A patch whose list overflows
-// (flat areas full of ties) and every patch of a tile whose samples overrun f16 goes through the exact
-// search of the whole window.
+// listed ones (nine or ten of 1,089 on noisy frames) in the exact order.
+//
+// Clean areas. Past 8 bits the samples are taken less the middle of the tile's, so that a tile of a narrow
+// range has exact scores whatever the depth, and lists real ties alone. A patch whose list still overflows
+// (hundreds of equal patches) and every patch of a tile whose samples overrun f16 falls back on exact
+// sums: where eight candidates seem to equal the patch, the window's first 48 until eight do (constant
+// areas); then the window in bands of rows, up to the first band that leaves eight equal patches in the
+// list. The groups without such a patch take a part of another's window. Streams of six frames, all
+// kernels, ms with the exact search of every candidate, with a full search per overflow, and so: 1080p
+// 8-bit r = 9 constant 22.0, 21.5, 15.8, dithered 32.6, 33.0, 25.2, flat shapes 24.1, 23.8, 18.8; 10-bit
+// 4:2:0 r = 16 constant 39.4, 46.6, 24.7, dithered 53.9, 62.8, 35.6, shapes 44.4, 52.5, 34.5 (noisy 43.3,
+// 25.4, 25.5). What gains least is a flat area with one sample in a hundred off, whose ties are not the
+// patch's equals and need every exact sum: 31.0, 31.3, 29.8 and 54.1, 62.7, 54.3; float chroma at 720p
+// 20.5, 22.1, 22.4.
 //
 // The error of a score, in units of squared codes: the tensor core's accumulation and the sums of squares
 // (screen_score.cuh, which also says what that rests on), the f32 distance's own rounding (1e-5 of it),
@@ -93,12 +104,6 @@ __device__ __forceinline__ void shift_insert8_key(const GroupCtx& g, float& best
     }
 }
 
-template <int C>
-__device__ __forceinline__ void load_row(float (&dst)[C], const float* __restrict__ colp, uint32_t row, int width) {
-#pragma unroll
-    for (int c = 0; c < C; ++c) dst[c] = __ldg(colp + static_cast<size_t>(row) * width * C + c);
-}
-
 // The group sums of eight candidates at once, each lane's eight column distances in `v`: the same
 // pairwise tree as reduce8 (partners xor 1, then 2, then 4), each level keeping half the candidates
 // on each side, so every total has the bits reduce8 gives it. Lane `sub` ends with the total of
@@ -126,44 +131,12 @@ __device__ __forceinline__ float reduce_scatter8(const GroupCtx& g, const float 
 
 __device__ __forceinline__ int scattered_candidate(int sub) { return (sub & 1) * 4 + (sub & 2) + ((sub >> 2) & 1); }
 
-// Eight candidate rows jb..jb+7 of window column `col` (the lane's sample column `colp`): `rows`
-// holds window rows jb..jb+6 on entry and jb+8..jb+14 on exit. Each candidate's distance is its
-// column sums in row order, the group's pairwise sum (reduce8's tree), times the channel scale;
-// the candidates that beat the list's worst key join it one at a time, in any order (the list is
-// the 8 smallest (distance, visiting index) pairs whatever the order they arrive in).
-template <int C>
-__device__ __forceinline__ void centre_batch(const GroupCtx& g, const float (&cur)[P * C], float (&rows)[15][C],
-                                             const float* __restrict__ colp, int width, uint32_t top, uint32_t jb,
-                                             uint32_t hh, uint32_t col, uint32_t ww, bool self_col,
-                                             uint32_t self_row, float scale, float& best_d, uint32_t& best_i,
-                                             float& worst_d, uint32_t& worst_i) {
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        if (jb + x < hh) {
-            load_row<C>(rows[7 + x], colp, top + jb + 7 + x, width);
-        } else {
-#pragma unroll
-            for (int c = 0; c < C; ++c) rows[7 + x][c] = 0.0f;
-        }
-    }
-    float v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        float sum = 0.0f;
-#pragma unroll
-        for (int r = 0; r < P; ++r)
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const float d = cur[r * C + c] - rows[k + r][c];
-                sum = __fadd_rn(sum, __fmul_rn(d, d));
-            }
-        v[k] = sum;
-    }
-    const uint32_t j = jb + static_cast<uint32_t>(scattered_candidate(g.sub));
-    float d = reduce_scatter8(g, v) * scale;
-    if (self_col && j == self_row) d = kSelfPin;
-    const uint32_t i = j * ww + col;
-    const bool wins = j < hh && d < kUnfilled && key_less(d, i, worst_d, worst_i);
+// One candidate per lane into the group's list, where `in` and it beats the list's worst key, one at a
+// time and in any order (the list is the 8 smallest (distance, visiting index) pairs whatever the order
+// they arrive in).
+__device__ __forceinline__ void take_winners(const GroupCtx& g, bool in, float d, uint32_t i, float& best_d,
+                                             uint32_t& best_i, float& worst_d, uint32_t& worst_i) {
+    const bool wins = in && d < kUnfilled && key_less(d, i, worst_d, worst_i);
     unsigned m = __ballot_sync(g.mask, wins) & g.mask;
     while (m) {
         const int src = __ffs(m) - 1;
@@ -176,33 +149,127 @@ __device__ __forceinline__ void centre_batch(const GroupCtx& g, const float (&cu
             worst_i = __shfl_sync(g.mask, best_i, 7, 8);
         }
     }
-#pragma unroll
-    for (int r = 0; r < 7; ++r)
-#pragma unroll
-        for (int c = 0; c < C; ++c) rows[r][c] = rows[8 + r][c];
 }
 
-
-// Every candidate of the clipped window in the exact order (fused/centre.rs:213-258), column by column,
-// eight candidate rows at a time with the column's rows in registers: one load per candidate and lane,
-// one reduce-scatter of the group per eight candidates.
+// A patch and its clipped window (fused/centre.rs:213-258). `cur` is the lane's column of the patch.
 template <int C>
-__device__ __noinline__ void centre_full(const GroupCtx& g, const float (&cur)[P * C], const float* __restrict__ centre,
-                                         int width, uint32_t rx, uint32_t ry, uint32_t left, uint32_t right,
-                                         uint32_t top, uint32_t bottom, float scale, float& best_d, uint32_t& best_i) {
-    const uint32_t ww = right - left + 1, hh = bottom - top + 1;
+struct PatchWindow {
+    float cur[P * C];
+    uint32_t rx, ry, left, top, ww, hh;
+    __device__ __forceinline__ uint32_t self() const { return (ry - top) * ww + (rx - left); }
+};
+
+template <int C>
+__device__ __forceinline__ PatchWindow<C> patch_window(const CollabLaunch& a, const float* __restrict__ centre,
+                                                       uint32_t rx, uint32_t ry, int sub) {
+    PatchWindow<C> p;
+    const uint32_t max_x = a.width - P, max_y = a.height - P;
+    const int R = a.spatial_radius;
+    p.rx = rx;
+    p.ry = ry;
+    p.left = clamp_top_left(static_cast<int>(rx) - R, max_x);
+    p.top = clamp_top_left(static_cast<int>(ry) - R, max_y);
+    p.ww = clamp_top_left(static_cast<int>(rx) + R, max_x) - p.left + 1;
+    p.hh = clamp_top_left(static_cast<int>(ry) + R, max_y) - p.top + 1;
+#pragma unroll
+    for (int r = 0; r < P; ++r)
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            p.cur[r * C + c] = __ldg(centre + ((static_cast<size_t>(ry) + r) * a.width + rx + sub) * C + c);
+    return p;
+}
+
+// The 8-lane group's list, one member per lane, and its worst key.
+struct TopEight {
+    float d = kUnfilled;
+    uint32_t i = 0xFFFFFFFFu;
     float worst_d = kUnfilled;
     uint32_t worst_i = 0xFFFFFFFFu;
-    for (uint32_t cx = left; cx <= right; ++cx) {
-        const float* colp = centre + static_cast<size_t>(cx + g.sub) * C;
-        const bool self_col = cx == rx;
-        const uint32_t col = cx - left, self_row = ry - top;
-        float rows[15][C];
+    // The patch itself, before any other candidate.
+    __device__ __forceinline__ void pin(const GroupCtx& g, uint32_t self) {
+        if (g.sub == 0) {
+            d = kSelfPin;
+            i = self;
+        }
+    }
+    __device__ __forceinline__ void take(const GroupCtx& g, bool in, float dist, uint32_t index) {
+        take_winners(g, in, dist, index, d, i, worst_d, worst_i);
+    }
+    // Eight candidates of which none can be beaten but by an earlier one.
+    __device__ __forceinline__ bool settled() const { return worst_d <= 0.0f; }
+};
+
+// The 15 samples a lane reads for eight candidate rows from window row jb of a column (rows past the
+// window's last repeat it), and the distance of candidate jb + scattered_candidate(sub): its column sums
+// in row order, the group's pairwise sum (reduce8's tree), times the channel scale.
+template <int C>
+struct ColumnBand {
+    float rows[15][C];
+    __device__ __forceinline__ void load(const PatchWindow<C>& p, const float* __restrict__ centre, int width,
+                                         uint32_t col, uint32_t jb, int sub) {
+        const float* colp = centre + static_cast<size_t>(p.left + col + sub) * C;
+        const uint32_t last = p.top + p.hh + P - 2;
 #pragma unroll
-        for (int r = 0; r < P - 1; ++r) load_row<C>(rows[r], colp, top + r, width);
-        for (uint32_t jb = 0; jb < hh; jb += 8)
-            centre_batch<C>(g, cur, rows, colp, width, top, jb, hh, col, ww, self_col, self_row, scale, best_d,
-                            best_i, worst_d, worst_i);
+        for (int r = 0; r < 15; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+                rows[r][c] = __ldg(colp + static_cast<size_t>(min(p.top + jb + r, last)) * width * C + c);
+    }
+    __device__ __forceinline__ float distance(const GroupCtx& g, const float (&cur)[P * C], float scale) const {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int r = 0; r < P; ++r)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    const float d = cur[r * C + c] - rows[k + r][c];
+                    sum = __fadd_rn(sum, __fmul_rn(d, d));
+                }
+            v[k] = sum;
+        }
+        return reduce_scatter8(g, v) * scale;
+    }
+};
+
+// Window columns [c0, c1) in the exact order, in bands of eight candidate rows. A band holds every earlier
+// visiting index than the next one's, so the search ends with the first that leaves the list settled.
+template <int C>
+__device__ __noinline__ TopEight centre_columns(const GroupCtx& g, const PatchWindow<C>& p,
+                                                const float* __restrict__ centre, int width, uint32_t c0,
+                                                uint32_t c1, float scale) {
+    TopEight best;
+    const uint32_t self_col = p.rx - p.left, self_row = p.ry - p.top;
+    if (self_col >= c0 && self_col < c1) best.pin(g, p.self());
+    for (uint32_t jb = 0; jb < p.hh && !best.settled(); jb += 8) {
+        const uint32_t j = jb + static_cast<uint32_t>(scattered_candidate(g.sub));
+        for (uint32_t col = c0; col < c1; ++col) {
+            ColumnBand<C> band;
+            band.load(p, centre, width, col, jb, g.sub);
+            best.take(g, j < p.hh && !(col == self_col && j == self_row), band.distance(g, p.cur, scale), j * p.ww + col);
+        }
+    }
+    return best;
+}
+
+// `n` candidates in the exact order, eight at a time: candidate k at the position `at(k)`. ORDERED: in
+// visiting order, and only until the list is settled.
+template <int C, bool ORDERED, class At>
+__device__ __forceinline__ void centre_listed(const GroupCtx& g, const PatchWindow<C>& p,
+                                              const float* __restrict__ centre, int width, int n, float scale, At at,
+                                              TopEight& best) {
+    for (int j0 = 0; j0 < n && !(ORDERED && best.settled()); j0 += 8) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint2 c = at(min(j0 + k, n - 1));
+            v[k] = column_ssd<C>(p.cur, centre, width, c.x, c.y, g.sub);
+        }
+        const int j = j0 + scattered_candidate(g.sub);
+        const float d = reduce_scatter8(g, v) * scale;
+        const uint2 c = at(min(j, n - 1));
+        best.take(g, j < n && !(c.x == p.rx && c.y == p.ry), d, (c.y - p.top) * p.ww + (c.x - p.left));
     }
 }
 
@@ -220,6 +287,8 @@ constexpr int kRefsX = 8, kRefsY = 4, kRefs = kRefsX * kRefsY;  // reference pat
 constexpr int kWarps = 8, kScreenThreads = 32 * kWarps;         // one 8-lane group per patch
 constexpr int kList = 48;                                       // candidates listed per patch
 constexpr int kShares = kWarps * 8;                             // shares of a patch's candidates
+constexpr int kProbe = 48;                                      // first candidates tried for eight equal ones
+constexpr int kMaxParts = 8;                                    // groups that share one window's columns
 constexpr int kMaxRadius = 16;
 constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
 constexpr float kOutside = -1e30f;
@@ -317,7 +386,28 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
     // spreads the 16-byte stores over the banks ----
     const bool codes = a.ring_code_max > 0.0f && a.ring_code_max <= 4095.0f;
     const float to_code = codes ? a.ring_code_max : 1023.0f;
-    const float mid = codes ? floorf(0.5f * a.ring_code_max + 0.5f) : 512.0f;
+    // What the samples are taken less. 8-bit codes: the middle of their range, where every score is exact.
+    // Others: the middle of 32 samples spread over the tile, per channel (every warp finds it for itself), a
+    // whole number, for codes one that leaves every code within the 2,048 that f16 holds exactly.
+    float mid[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) mid[c] = 128.0f;
+    if (!codes || to_code > 255.0f) {
+        const int gx = min(max(ox - R + (lane & 7) * (16 * tiles + 6) / 7, 0), a.width - 1);
+        const int gy = min(max(oy - R + (lane >> 3) * (rows - 1) / 3, 0), a.height - 1);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            float lo = __ldg(centre + (static_cast<size_t>(gy) * a.width + gx) * C + c), hi = lo;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            }
+            const float m = rintf(0.5f * (lo + hi) * to_code);
+            mid[c] = fabsf(m) <= 65536.0f ? m : 512.0f;  // NaN and infinities: the tile is searched in full
+            if (codes) mid[c] = fminf(fmaxf(mid[c], to_code - 2048.0f), 2048.0f);
+        }
+    }
     float worst = 0.0f;
     bool bad = false;
     const int segs = 2 * tiles;
@@ -337,8 +427,8 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
             for (int c = 0; c < C; ++c) {
                 const float s = __ldg(src + static_cast<size_t>(gx) * C + c);
                 // codes: rounded to the code; floats: rounded to f16
-                const float x = codes ? fmaf(s, to_code, kRound - mid) - kRound
-                                      : __half2float(__float2half_rn(fmaf(s, to_code, -mid)));
+                const float x = codes ? fmaf(s, to_code, kRound - mid[c]) - kRound
+                                      : __half2float(__float2half_rn(fmaf(s, to_code, -mid[c])));
                 bad |= !(fabsf(x) <= 2048.0f);
                 worst = fmaxf(worst, fabsf(x));
                 v[c][i] = x;
@@ -374,7 +464,10 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
 #pragma unroll
         for (int i = 0; i < 8; ++i) squares[y * cp + x0 + i] = part[i];
     }
+    __shared__ int pending[kRefs], npending;
+    __shared__ bool even[kRefs];  // eight candidates may equal the patch
     if (tid < kRefs) count[tid] = 0;
+    if (tid == 0) npending = 0;
     bad = __syncthreads_or(bad);
     for (int task = tid; task < ((crows + 7) / 8) * 16 * tiles; task += kScreenThreads) {
         const int run_y = task / (16 * tiles), x = task - run_y * 16 * tiles;
@@ -399,6 +492,7 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
     // The group's patch (column n of the instruction) and this thread's two (columns 2 t4, 2 t4 + 1), as
     // positions in the tile: a patch's window starts at its own position less the tile's first patch.
     const uint32_t chunk_addr = static_cast<uint32_t>(__cvta_generic_to_shared(chunks));
+    bool over = bad;  // some list of the CTA overflowed, or there are none
     if (!bad) {
         uint32_t b[4][8 * C];
         int px[4][2], py[4], first_x[2], last_x[2], first_y[2], last_y[2];
@@ -486,13 +580,16 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
                 const float n = 64.0f * C;
                 const float reach = 3.0f * n * worst * worst;  // no partial sum is larger
                 const float dist = fmaxf(-sums[qy * cp + qx] - eighth, 0.0f);
-                const float fixed = 4.0f + screen::score_error<C>(reach);
+                // Codes below kExactBelow have whole scores: an allowance under a half keeps to real ties.
+                const float fixed = (codes ? 1e-3f : 4.0f) + screen::score_error<C>(reach);
                 const float dist1 = dist + fixed;
                 // |D - D~| <= 2 sqrt(D) times the norm of the quotients' rounding, 2 * 2^-24 to_code a sample.
                 const float quotients = (codes ? 4.0f * screen::kUlp * to_code * sqrtf(n * dist1) : 0.0f) + 1e-5f * dist1;
-                const float halves = codes ? 0.0f : 2.0f * sqrtf(n) * worst * 4.9e-4f;
+                // f16 rounds at 2^-11 of the sample, and at 2^-25 near zero.
+                const float halves = codes ? 0.0f : 2.0f * sqrtf(n) * (worst * 4.9e-4f + 3e-8f);
                 const float slack = 2.0f * (fixed + quotients) + 4.0f * halves * (sqrtf(dist1) + halves);
                 line[ref] = fmaxf(eighth - slack, -1e29f);
+                even[ref] = dist <= fixed;
             }
         }
         __syncthreads();
@@ -510,72 +607,78 @@ __global__ void __launch_bounds__(kScreenThreads, C == 1 ? 2 : 1) collab_screen_
                                if (s0 >= bar[nt][e]) {
                                    const int at = atomicAdd(count + ref, 1);
                                    if (at < kList) list[ref * kList + at] = static_cast<uint16_t>(cell);
+                                   over |= at >= kList;
                                }
                                if (s1 >= bar[nt][e]) {
                                    const int at = atomicAdd(count + ref, 1);
                                    if (at < kList) list[ref * kList + at] = static_cast<uint16_t>(cell + 8);
+                                   over |= at >= kList;
                                }
                            }
                        });
-        __syncthreads();
+        over = __syncthreads_or(over);
     }
 
     // ---- the listed candidates in the exact order, one 8-lane group per patch ----
     GroupCtx g;
     g.sub = tid & 7;
     g.mask = 0xFFu << (lane & ~7);
-    const int ref = tid >> 3;
-    const int ix = ix0 + ref % kRefsX, iy = iy0 + ref / kRefsX;
-    if (ix >= refs_x || iy >= refs_y) return;  // the group's 8 lanes leave together; no barrier follows
-    const uint32_t rx = min(ix * STEP, max_x), ry = min(iy * STEP, max_y);
+    const int group = tid >> 3;
     const float scale = C == 1 ? 3.0f : 1.5f;
-    float cur[P * C];
-#pragma unroll
-    for (int r = 0; r < P; ++r)
-#pragma unroll
-        for (int c = 0; c < C; ++c)
-            cur[r * C + c] = __ldg(centre + ((static_cast<size_t>(ry) + r) * a.width + rx + g.sub) * C + c);
-    const uint32_t left = clamp_top_left(static_cast<int>(rx) - R, max_x);
-    const uint32_t right = clamp_top_left(static_cast<int>(rx) + R, max_x);
-    const uint32_t top_row = clamp_top_left(static_cast<int>(ry) - R, max_y);
-    const uint32_t bottom = clamp_top_left(static_cast<int>(ry) + R, max_y);
-    const uint32_t ww = right - left + 1, hh = bottom - top_row + 1;
-    float best_d = kUnfilled, worst_d = kUnfilled;
-    uint32_t best_i = 0xFFFFFFFFu, worst_i = 0xFFFFFFFFu;
-    const int listed = bad ? kList + 1 : count[ref];
-    if (listed > kList) {
-        centre_full<C>(g, cur, centre, a.width, rx, ry, left, right, top_row, bottom, scale, best_d, best_i);
-    } else {
-        for (int j0 = 0; j0 < listed; j0 += 8) {
-            float v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int cell = list[ref * kList + min(j0 + k, listed - 1)];
-                v[k] = column_ssd<C>(cur, centre, a.width, ox - R + (cell & 63), oy - R + (cell >> 6), g.sub);
-            }
-            const int j = j0 + scattered_candidate(g.sub);
-            float d = reduce_scatter8(g, v) * scale;
-            const int cell = list[ref * kList + min(j, listed - 1)];
-            const uint32_t cx = ox - R + (cell & 63), cy = oy - R + (cell >> 6);
-            if (cx == rx && cy == ry) d = kSelfPin;
-            const uint32_t i = (cy - top_row) * ww + (cx - left);
-            const bool wins = j < listed && d < kUnfilled && key_less(d, i, worst_d, worst_i);
-            unsigned m = __ballot_sync(g.mask, wins) & g.mask;
-            while (m) {
-                const int src = __ffs(m) - 1;
-                m &= m - 1;
-                const float dd = __shfl_sync(g.mask, d, src);
-                const uint32_t ii = __shfl_sync(g.mask, i, src);
-                if (key_less(dd, ii, worst_d, worst_i)) {  // uniform: every lane holds the same words
-                    shift_insert8_key(g, best_d, best_i, dd, ii);
-                    worst_d = __shfl_sync(g.mask, best_d, 7, 8);
-                    worst_i = __shfl_sync(g.mask, best_i, 7, 8);
-                }
-            }
+    auto window_of = [&](int ref) {
+        return patch_window<C>(a, centre, min((ix0 + ref % kRefsX) * STEP, max_x), min((iy0 + ref / kRefsX) * STEP, max_y),
+                               g.sub);
+    };
+    auto write = [&](int ref, const PatchWindow<C>& p, const TopEight& best) {
+        const int ix = ix0 + ref % kRefsX, iy = iy0 + ref / kRefsX;
+        write_members(g, a.members + static_cast<size_t>(iy * refs_x + ix) * kMemberWords, best.i, p.left, p.top, p.ww,
+                      p.hh, a.k_max);
+    };
+    if (ix0 + group % kRefsX < refs_x && iy0 + group / kRefsX < refs_y) {
+        const PatchWindow<C> p = window_of(group);
+        TopEight best;
+        best.pin(g, p.self());
+        const int listed = bad ? kList + 1 : count[group];
+        if (listed <= kList) {
+            centre_listed<C, false>(g, p, centre, a.width, listed, scale,
+                                    [&](int k) {
+                                        const int cell = list[group * kList + k];
+                                        return make_uint2(ox - R + (cell & 63), oy - R + (cell >> 6));
+                                    },
+                                    best);
+        } else {
+            const int probe = bad || even[group] ? min(static_cast<int>(p.ww * p.hh), kProbe) : 0;
+            centre_listed<C, true>(g, p, centre, a.width, probe, scale,
+                                   [&](int k) { return make_uint2(p.left + k % p.ww, p.top + k / p.ww); }, best);
         }
+        if (listed <= kList || best.settled()) write(group, p, best);
+        else if (g.sub == 0) pending[atomicAdd(&npending, 1)] = group;
     }
-    write_members(g, a.members + static_cast<size_t>(iy * refs_x + ix) * kMemberWords, best_i, left, top_row, ww, hh,
-                  a.k_max);
+    if (!over) return;  // the same for the whole CTA
+
+    // ---- the patches left: each window's columns in as many parts as there are groups for it ----
+    __syncthreads();
+    const int n = npending;
+    if (n == 0) return;
+    const int parts = min(kRefs / n, kMaxParts), part = group / n;
+    struct Member {
+        float d;
+        uint32_t i;
+    };
+    Member* found = reinterpret_cast<Member*>(squares);  // [kRefs][8]
+    TopEight best;
+    if (part < parts) {
+        const PatchWindow<C> p = window_of(pending[group % n]);
+        best = centre_columns<C>(g, p, centre, a.width, p.ww * part / parts, p.ww * (part + 1) / parts, scale);
+        found[group * 8 + g.sub] = Member{best.d, best.i};
+    }
+    __syncthreads();
+    if (part > 0) return;
+    for (int q = 1; q < parts; ++q) {
+        const Member m = found[(group + q * n) * 8 + g.sub];
+        best.take(g, true, m.d, m.i);
+    }
+    write(pending[group], window_of(pending[group]), best);
 }
 
 // One block of a refine rectangle: up to 5 x 5 candidates from (x0, y0), each scored in the exact order.

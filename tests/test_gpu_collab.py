@@ -132,13 +132,22 @@ def screen_frame(kind: str, w: int, h: int, c: int, rng) -> np.ndarray:
         base[h // 3, w // 3] = 1e5
     elif kind == "codes":
         base = np.round(np.clip(base, 0, 1) * 255) / 255
+    elif kind == "specks":  # some patches overflow with equal candidates that are not the patch's own
+        base = 0.25 + (rng.uniform(size=(h, w, c)) < 0.02) * 0.01
+    elif kind == "ramp":  # equal patches in every row, too few in one
+        base = np.broadcast_to(np.floor(x / 3)[..., None] / 128, (h, w, c)).copy()
+    elif kind == "tiny":  # steps that f16 rounds near its smallest numbers
+        base = 0.5 + rng.integers(-3, 4, (h, w, c)) * 2.0 ** -24
     return base.astype(np.float32)
 
 
 @pytest.mark.parametrize("kind,w,h,c,sr", [("noise", 8, 8, 1, 16), ("noise", 9, 10, 2, 3), ("noise", 75, 43, 1, 16),
                                            ("codes", 61, 70, 2, 16), ("noise", 41, 25, 1, 1), ("flat", 64, 48, 1, 9),
                                            ("levels", 66, 37, 1, 7), ("levels", 48, 48, 2, 12),
-                                           ("wide", 70, 52, 1, 9), ("wide", 40, 36, 2, 5)])
+                                           ("wide", 70, 52, 1, 9), ("wide", 40, 36, 2, 5),
+                                           ("flat", 50, 70, 2, 16), ("specks", 83, 61, 1, 16), ("specks", 52, 45, 2, 9),
+                                           ("ramp", 90, 40, 1, 12), ("ramp", 44, 66, 2, 6), ("tiny", 60, 41, 1, 9),
+                                           ("flat", 9, 33, 1, 2), ("specks", 36, 20, 2, 1)])
 def test_screened_search_picks_the_exact_members(oracle, kind, w, h, c, sr):
     """The centre search scores candidates on the tensor cores and settles the best eight in the exact
     order: tile and frame edges, one patch, lists that overflow and samples past f16, every accumulator

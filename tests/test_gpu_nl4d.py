@@ -78,6 +78,43 @@ def test_nl4d_deep_codes(oracle, depth):
         assert np.array_equal(g[0], wn[0])
 
 
+def clean_planes(kind, w, h, n, depth, rng):
+    """Frames without noise, or next to none: ties by the hundred among the candidates of a search."""
+    top = (1 << depth) - 1
+    y, x = np.mgrid[0:h, 0:w]
+    base = np.full((h, w), top // 6)
+    frames = []
+    for k in range(n):
+        f = base.copy()
+        if kind == "specks":  # a few samples off by little
+            f = f + (rng.uniform(size=(h, w)) < 0.01) * 3
+        elif kind == "dither":
+            f = f + np.round(rng.normal(0, 0.4, (h, w))).astype(int)
+        elif kind == "ramp":  # equal columns
+            f = f + x // 3
+        elif kind == "shapes":  # flat areas with edges in both directions, moving
+            f = np.where((x - k) % 40 < 17, top // 2, f) + ((y + k) % 31 < 12) * (top // 3)
+        elif kind == "letterbox":
+            f[h // 4:-(h // 4)] = rng.integers(0, top + 1, (h - 2 * (h // 4), w))
+        frames.append(np.clip(f, 0, top).astype(np.uint8 if depth == 8 else np.uint16))
+    return frames
+
+
+@pytest.mark.parametrize("kind", ["constant", "specks", "dither", "ramp", "shapes", "letterbox"])
+@pytest.mark.parametrize("depth,sr", [(8, 9), (10, 16), (12, 5)])
+def test_nl4d_clean_frames(oracle, kind, depth, sr):
+    """Ties past what a patch's list holds: the first candidates, the bands of rows and the parts of a window
+    that other groups search keep the members of the full search."""
+    w, h, d, sigma = 100, 62, 1, 8.0 / 255
+    fmt = avd.SampleFormat.u8() if depth == 8 else avd.SampleFormat.u16(depth)
+    rng = np.random.default_rng(depth + len(kind))
+    frames = [[f] for f in clean_planes(kind, w, h, 4, depth, rng)]
+    spec = avd.EngineSpec.nl4d(opts(d, sigma, spatial_radius=sr), None,
+                               avd.Geometry(w, h, avd.ChromaLayout.GRAY, fmt, fmt))
+    got = Runner(spec).run(frames)
+    check(oracle, got, frames, fmt, d, sigma, spatial_radius=sr)
+
+
 def test_nl4d_plain_threshold_10bit(oracle):
     w, h, d, sigma = 64, 48, 1, 8.0 / 255
     fmt = avd.SampleFormat.u16(10)
