@@ -80,6 +80,8 @@ struct NlmLaunch {
 };
 
 cudaError_t launch_nlm(const NlmLaunch& args, cudaStream_t stream);
+// The column-pair tile is built for the patch radii up to the default. It gains at 5 as well (1080p luma d = 2
+// a = 5: 1,410 us on the offset-pair tile, 1,187 on it; a = 2: 331 and 288), which is not built yet.
 constexpr int kColsMaxPatch = 4;
 // The column-pair tile, `split` CTAs of a cluster to a tile, without (fast) and with noise offsets, in
 // the resident CTAs of args.variant.
@@ -108,12 +110,14 @@ cudaError_t launch_nlm_exact(const NlmLaunch& args, cudaStream_t stream, int* ti
 cudaError_t launch_exp_mirror(const float* x, float* out, int64_t n, cudaStream_t stream);
 // The band the window kernel flags around each rounding boundary, in normalised units:
 // kFixBand + kFixBandPerH2 * h2. The window kernel's float result differs from the mirror's by the
-// box sums' and the MUFU exponential's rounding, which the strength h2 amplifies. Measured over
-// strengths 1..16, patch radii 1..3, luma, chroma and NLMeans-HQ: the 99.99th percentile of the
-// difference lies inside the band everywhere (6e-7 against 2.07e-6 at the 1080p luma workload's
-// h2 of 13.5; 3.4e-6 against 1.4e-5 at h2 2408), the largest difference inside it where h2 is
-// below 30. A sample is missed only where a difference past the band meets a value that close to a
-// boundary: a few in ten million.
+// box sums' and the MUFU exponential's rounding, which the strength h2 amplifies. Measured on the
+// column-pair tile (the offset-pair tile's figures are the same or larger) over patch radii 0..4,
+// search radii 2..8, d 0..4, strengths 1.2, 4 and 12, luma, chroma and NLMeans-HQ, 8 and 10 bits, 1.2
+// billion samples: on noisy frames the 99.99th percentile of the difference is 0.76 of the band at most
+// and the largest difference three bands (but for a pixel whose weights all underflow); on frames cut
+// by hard edges (codes 3 and 252, little noise) 3.2 bands and 7.6 at strength 1.2. A sample is missed
+// only where a difference past the band meets a value that close to a boundary: 2 of 830 million on
+// the noisy frames, 111 of 410 million on the edges (93 of them at strength 1.2).
 constexpr float kFixBand = 2e-6f;
 constexpr float kFixBandPerH2 = 5e-9f;
 // The same launch with `args.ref_ring` set (prefilter.cu).

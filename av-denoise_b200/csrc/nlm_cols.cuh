@@ -21,7 +21,8 @@
 // 0.288 -> 0.271 ms. Small frames share a tile between the CTAs of a cluster (cols_split, nlm.cu).
 //
 // The order of every sum within a distance is the one of nlm_tile.cuh (runs from multiples of 8
-// columns, strips of V rows), so the distances keep their bits.
+// columns, strips of V rows). The samples are staged less a level (tile_level), which rounds those
+// darker than it, so a distance may differ from that tile's in its last bits.
 
 #pragma once
 
@@ -267,10 +268,12 @@ __device__ __forceinline__ void cols_frame(ColsState<C, K>& z, int A, int dy0, i
     }
 }
 
-// The level samples are staged relative to, per channel: just under the tile's darkest pixel. The weighted
-// sum is then of smaller values and keeps bits that one running sum over several hundred offsets would
-// lose, dark pixels' included. The level is a multiple of 1/256 below the samples, so the subtraction is
-// exact and the distances do not change. `two` is shared memory for two pairs; every thread calls it.
+// The level samples are staged relative to, per channel: just under the darkest pixel the tile owns. The
+// weighted sum is then of smaller values and keeps bits that one running sum over several hundred offsets
+// would lose, dark pixels' included. The level is a multiple of 1/256, so the subtraction is exact for
+// samples at or above it. Darker ones (beside the tile, or in another frame) are rounded by up to 2^-25 =
+// 3e-8, a sixtieth of the exact finish's band; the band's measurement (kernels.h) has hard edges in it.
+// `two` is shared memory for two pairs; every thread calls it.
 template <int C, class K>
 __device__ __forceinline__ float2 tile_level(const float* __restrict__ centre, int X0, int Y0, int W, int H, float2* two) {
     const int tid = threadIdx.x, col = tid & (kHalf - 1), y0 = (tid / kHalf) * K::V;

@@ -249,8 +249,8 @@ def run_gpu(args) -> None:
         (n, _), t = timed(step_device)
         assert n == FRAMES
         times.append(t)
+        nlm_timing = eng_l.timing().luma  # window kernel + exact finish per luma frame, before its counts run over
     wall = time.perf_counter() - wall0
-    nlm_timing = eng_l.timing().luma  # window kernel + exact finish per luma frame
     eng_l.sample_device_time(0)
     # The chroma engine's frame, sampled on one more (untimed) step so the timed steps carry only
     # the luma engine's sampling events.
@@ -382,6 +382,7 @@ def run_gpu(args) -> None:
     t_luma_frame = nlm_timing.device_time / max(1, nlm_timing.frames)
     achieved = ex2_per_launch / t_window / 1e9
     mufu_peak = sms * 16 * peaks["sm_max_mhz"] * 1e6 / 1e9
+    smem_peak = 8 * mufu_peak  # 128 bytes against 16 exponentials per clock and SM
     hbm_bytes = luma_px * 4 * (2 * LUMA["d"] + 1) + luma_px * 4
     line = {
         "metric": METRIC,
@@ -400,15 +401,17 @@ def run_gpu(args) -> None:
                                "chroma spatial a=5 s=2 strength 5 (a luma engine and a chroma engine on two "
                                "streams)", "frames_per_step": FRAMES,
                    "l2": "flushed between steps (256 MiB write)", "parallelism": f"replicas x{world}"},
-        "roofline": {"bound": "sfu", "kernel": "nlm_cols_kernel<1,2,fast> (luma, 604 offsets/pixel)",
-                     "achieved": round(achieved, 2), "peak": round(mufu_peak, 2), "unit": "Gex2/s",
-                     "frac": round(achieved / mufu_peak, 4),
+        # The box sums cross threads through shared memory: 17.5 bytes per (pixel, offset) at s = 2.
+        "roofline": {"bound": "shared memory", "kernel": "nlm_cols_kernel<1,2,fast> (luma, 604 offsets/pixel)",
+                     "achieved": round(achieved * 17.5, 1), "peak": round(smem_peak, 1), "unit": "GB/s",
+                     "frac": round(achieved * 17.5 / smem_peak, 4),
                      # dram__bytes_read.sum + dram__bytes_write.sum of one launch in an ncu capture of
                      # the same launch, not of this run.
-                     "traffic": 41.52e6 + 0.151e6,
-                     "traffic_source": "ncu capture: profiles/nlm_window_kernel_luma_1080p_d2a5s2.md",
-                     "peak_note": f"MUFU ex2: {sms} SMs x 16/clk x sm_max_mhz {peaks['sm_max_mhz']} "
-                                  f"({peaks['source']})",
+                     "traffic": 41.84e6 + 0.097e6,
+                     "traffic_source": "ncu capture: profiles/window_and_search_kernels_1080p.md",
+                     "peak_note": f"{sms} SMs x 128 B/clk x sm_max_mhz {peaks['sm_max_mhz']} ({peaks['source']})",
+                     "exponentials": {"achieved": round(achieved, 2), "peak": round(mufu_peak, 2), "unit": "Gex2/s",
+                                      "frac": round(achieved / mufu_peak, 4)},
                      "launch_ms": round(t_window * 1e3, 4),
                      "luma_frame_ms_with_exact_finish": round(t_luma_frame * 1e3, 4),
                      # pixels per luma frame the exact finish recomputed in the reference's order
@@ -513,34 +516,25 @@ def nl4d_4k_section(avd, torch, np, synth, pushes: int) -> dict:
     steady = times[fill:]
     ms = float(np.median(steady))
 
-    # The group search's algorithmic FP32 operations per launch: every reference patch's clipped
-    # centre window (33 x 33 inside the frame) and at least one 5 x 5 refine rectangle per volume
-    # and neighbour frame, each candidate 64 squared differences per channel (sub, mul, add: the
-    # oracle's unfused order) plus the group sum and the scale (8).
-    def search_ops(pw, ph, c):
+    # The candidates of the centre windows (33 x 33, clipped to the frame), which the screen scores.
+    def centre_candidates(pw, ph):
         def axis(n):
             top = n - 8
             return sum(min(min(i * 4, top) + 16, top) - max(min(i * 4, top) - 16, 0) + 1
                        for i in range((top + 3) // 4 + 1))
-        refs = ((pw - 8 + 3) // 4 + 1) * ((ph - 8 + 3) // 4 + 1)
-        per_candidate = 64 * c * 3 + 8
-        return (axis(pw) * axis(ph) + refs * 2 * (2 * d) * 25) * per_candidate
+        return axis(pw) * axis(ph)
 
-    unfused_rate = 148 * 128 * 1.965e9  # FP32 lanes x the B200's top SM clock: one operation per lane per clock
     core = {}
-    for name, t, (pw, ph), c in (("luma", timing.luma, dims[0], 1), ("chroma", timing.chroma, dims[1], 2)):
+    for name, t, (pw, ph) in (("luma", timing.luma, dims[0]), ("chroma", timing.chroma, dims[1])):
         if t is None or t.core_launches == 0:
             continue
-        launch_s = t.core_time / t.core_launches
-        ops = search_ops(pw, ph, c)
-        core[name] = {"launch_ms": round(launch_s * 1e3, 3), "search_gops": round(ops / 1e9, 1),
-                      "achieved_tops": round(ops / launch_s / 1e12, 2),
-                      "frac_unfused_fp32": round(ops / launch_s / unfused_rate, 3)}
+        core[name] = {"ms_per_pass": round(t.core_time / t.core_launches * 1e3, 3),
+                      "centre_candidates": centre_candidates(pw, ph)}
     return {"workload": "NL4D 3840x2160 4:2:0 10-bit luma+chroma, d=3 (Chained), spatial_radius 16, lambda_ht 2.7, "
                         "plain threshold; sigma automatic on both plane groups, noise map and colour gains on",
             "frames_per_s": round(1000.0 / ms, 2), "ms_per_frame": round(ms, 3), "pushes_timed": len(steady),
-            "group_search": dict(core, note="CUDA events around each steady-state pass's group search + filter "
-                                            "launch; operations counted for the search alone, so a lower bound")}
+            "search_and_filter": dict(core, note="CUDA events around each steady-state pass's group search "
+                                                 "(screen and walk) and filter launches")}
 
 
 def run_reference(args) -> None:
