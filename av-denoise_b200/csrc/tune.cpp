@@ -91,11 +91,19 @@ void append(const std::string& dir, const std::string& key, int variant, const s
 
 std::string tune_device_identity() {
     int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return "unknown";
+    // The query takes milliseconds, and every engine asks at its first window: once per device.
+    static std::mutex lock;
+    static std::map<int, std::string> known;
+    std::lock_guard<std::mutex> g(lock);
+    std::string& id = known[dev];
+    if (!id.empty()) return id;
     cudaDeviceProp p{};
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaGetDeviceProperties(&p, dev) != cudaSuccess) return "unknown";
-    std::ostringstream id;
-    id << p.name << " sm_" << p.major << p.minor << " x" << p.multiProcessorCount;
-    return id.str();
+    if (cudaGetDeviceProperties(&p, dev) != cudaSuccess) return "unknown";
+    std::ostringstream text;
+    text << p.name << " sm_" << p.major << p.minor << " x" << p.multiProcessorCount;
+    id = text.str();
+    return id;
 }
 
 int tuned_variant(const TuneOptions& options, const std::string& key, int variants,

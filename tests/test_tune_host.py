@@ -75,3 +75,52 @@ def test_tuning_config_maps_onto_the_abi():
     assert t.mode == CACHED and t.store == b"/tmp/x" and t.deterministic == 0
     with pytest.raises(avd.InvalidOptions):
         avd.TuningConfig(mode="sometimes")._c()
+
+
+IDENTITY_PROGRAM = r"""
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <cuda_runtime.h>
+#include "tune.h"
+
+static int current = 0, queries = 0, fail = 0;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = current; return cudaSuccess; }
+extern "C" cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int dev) {
+    ++queries;
+    if (fail) return cudaErrorInvalidValue;
+    std::snprintf(p->name, sizeof(p->name), "GPU %d", dev);
+    p->major = 10;
+    p->minor = 0;
+    p->multiProcessorCount = 100 + dev;
+    return cudaSuccess;
+}
+
+int main() {
+    fail = 1;
+    if (avd::tune_device_identity() != "unknown") return 1;
+    fail = 0;
+    for (int round = 0; round < 3; ++round)
+        for (int dev : {0, 3}) {
+            current = dev;
+            if (avd::tune_device_identity() != "GPU " + std::to_string(dev) + " sm_100 x" + std::to_string(100 + dev))
+                return 2;
+        }
+    return queries == 3 ? 0 : 3;  // the one that failed, then one per device
+}
+"""
+
+
+def test_the_device_is_identified_once(tmp_path):
+    """The properties query takes milliseconds, and every engine asks for its store key at its first
+    window: one query per device, against a stand-in of the runtime."""
+    import subprocess
+    from pathlib import Path
+
+    root = Path(__file__).resolve().parent.parent
+    csrc = root / "av-denoise_b200" / "csrc"
+    src, exe = tmp_path / "identity.cpp", tmp_path / "identity"
+    src.write_text(IDENTITY_PROGRAM)
+    subprocess.run(["g++", "-std=c++17", f"-I{csrc}", f"-I{root / 'include'}", "-I/usr/local/cuda/include", str(src),
+                    str(csrc / "tune.cpp"), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
