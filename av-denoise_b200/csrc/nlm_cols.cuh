@@ -361,7 +361,7 @@ __device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int ti
     const int cols = kHalf + 2 * S + 2 * A, side = 2 * A + 1;
     const int all = (2 * a.pairs + 1) * side;  // window rows of the whole tile
     float2* kept = hs + K::HS_PAIRS + tid;  // [(C + 1) V] of this thread, kColsThreads apart
-    int share = CLUSTER ? rank : 0;
+    int share = CLUSTER ? rank : 0, held = -1;  // the frame the tile holds
     for (int step = 0; step <= 2 * a.pairs || (!CLUSTER && share + 1 < split); ++step) {
         if (step > 2 * a.pairs) {  // the next share, from the centre frame on
             keep_sums<C, K>(z, kept, share == 0);
@@ -379,8 +379,11 @@ __device__ __forceinline__ void cols_tile(const NlmLaunch& a, int tile_x, int ti
         // The forward's order: pair by pair and offset by offset, the forward frame at q (an even id),
         // then the backward frame at -q; the single-frame pass last.
         const int id_first = 2 * pair * side * side + (fwd ? 0 : 2 * side * side - 1), id_step = fwd ? 2 : -2;
-        load_cols<K, C>(tile, a.ring + slot * a.frame_elems, X0 - S - A, Y0 - S - A, K::rows(A), cols, W, H, mu);
-        __syncthreads();
+        if (CLUSTER || REC || f != held) {  // the next share may begin in the frame the last one ended in
+            load_cols<K, C>(tile, a.ring + slot * a.frame_elems, X0 - S - A, Y0 - S - A, K::rows(A), cols, W, H, mu);
+            __syncthreads();
+            held = f;
+        }
         if (f == 0) {
 #pragma unroll
             for (int i = 0; i < K::RUNW; ++i) z.ctr[i] = load_pair<C>(z.run + i * C);
